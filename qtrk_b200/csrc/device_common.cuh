@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "qtrk_c_api.h"
 #include "track_params.h"
 
 namespace qtrk {
@@ -52,6 +53,7 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double *red)
 
 // Thread groups that process one ROI: the whole CTA, or one warp (small-ROI kernels).
 struct BlockGroup {
+    static constexpr int kFold = 64;  // pixels per FP32 partial sum of the COM
     double *red;  // >= N*32 doubles of shared scratch for sum<N>
     __device__ __forceinline__ int rank() const { return threadIdx.x; }
     __device__ __forceinline__ int size() const { return blockDim.x; }
@@ -60,17 +62,24 @@ struct BlockGroup {
     __device__ __forceinline__ void sum(double (&v)[N]) const { block_sum<N>(v, red); }
 };
 
-struct WarpGroup {
-    __device__ __forceinline__ int rank() const { return threadIdx.x & 31; }
-    __device__ __forceinline__ int size() const { return 32; }
-    __device__ __forceinline__ void sync() const { __syncwarp(); }
+// kLanes (16 or 32) consecutive lanes of a warp.
+template <int kLanes>
+struct LaneGroup {
+    static constexpr int kFold = 8;
+    __device__ __forceinline__ unsigned mask() const
+    {
+        return kLanes == 32 ? 0xffffffffu : ((1u << (kLanes & 31)) - 1u) << (threadIdx.x & 31 & ~(kLanes - 1));
+    }
+    __device__ __forceinline__ int rank() const { return threadIdx.x & (kLanes - 1); }
+    __device__ __forceinline__ int size() const { return kLanes; }
+    __device__ __forceinline__ void sync() const { __syncwarp(mask()); }
     template <int N>
     __device__ __forceinline__ void sum(double (&v)[N]) const
     {
 #pragma unroll
         for (int k = 0; k < N; k++)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+            for (int o = kLanes / 2; o > 0; o >>= 1) v[k] += __shfl_xor_sync(mask(), v[k], o);
     }
 };
 
@@ -257,6 +266,35 @@ __device__ __forceinline__ int warp_argmax(Get at, int len)
     return bi < 0 ? 0 : bi;
 }
 
+// The words of job i (frame i and zeros without a job array) and the 13 words of a result.
+__device__ __forceinline__ void read_job(const LocalizationJob *jobs, int i, uint32_t (&w)[6])
+{
+    if (jobs) {
+        const uint32_t *p = reinterpret_cast<const uint32_t *>(jobs) + (size_t)i * 6;
+#pragma unroll
+        for (int k = 0; k < 6; k++) w[k] = p[k];
+    } else {
+        w[0] = (uint32_t)i;
+#pragma unroll
+        for (int k = 1; k < 6; k++) w[k] = 0;
+    }
+}
+
+__device__ __forceinline__ void write_result(LocalizationResult *results, int i, const uint32_t (&job)[6], float x,
+                                             float y, float z, float gx, float gy, uint32_t err, float mean)
+{
+    uint32_t *o = reinterpret_cast<uint32_t *>(results) + (size_t)i * 13;
+#pragma unroll
+    for (int k = 0; k < 6; k++) o[k] = job[k];
+    o[6] = __float_as_uint(x);
+    o[7] = __float_as_uint(y);
+    o[8] = __float_as_uint(z);
+    o[9] = __float_as_uint(gx);
+    o[10] = __float_as_uint(gy);
+    o[11] = err;
+    o[12] = __float_as_uint(mean);
+}
+
 // -------------------------------------------------------------------------------------
 // ROI load: u8/u16/f32 -> f32 tile in shared memory, with the clear-first-four-pixels
 // option (QueuedCPUTracker.cpp:280-282) and the per-bead offset/gain step
@@ -376,34 +414,54 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
         }
     } else {
         // Rows at a pitch (a ROI inside a frame): warps over rows, lanes along a row, so loads
-        // are coalesced along the row and the stores are conflict-free.
-        // With whole 4-pixel chunks the partial sums are then taken from the tile in the chunk
+        // are coalesced along the row and the stores are conflict-free. Rows back to back that are
+        // not whole aligned 16-byte units (odd ROI sizes) are one flat run, loaded in batches of
+        // eight so that the latency is paid per batch and not per row.
+        // The partial sums are then taken from the tile, with whole 4-pixel chunks in the chunk
         // order of the contiguous loads, so that a ROI gives bit-identical results whichever way
         // it arrived (FP32 partial sums depend on which pixels each thread adds).
         const bool chunked = !(n & 3) && !(reinterpret_cast<uintptr_t>(img) & 15);
-        const int lane = g.rank() & 31, wg = g.rank() >> 5, nwg = g.size() >> 5;
-        for (int y = wg; y < H; y += nwg) {
-            const uint8_t *row = src + (size_t)y * pitch;
-#pragma unroll 4
-            for (int x = lane; x < W; x += 32) {
-                float v;
-                if (P.pdt == 0)
-                    v = u_to_float(row[x]);
-                else if (P.pdt == 1)
-                    v = u_to_float(reinterpret_cast<const uint16_t *>(row)[x]);
-                else
-                    v = reinterpret_cast<const float *>(row)[x];
-                const int i = y * W + x;
-                v = finish_pixel(v, i, P, off, gain);
-                if (!chunked) {
-                    s += v;
-                    s2 = fmaf(v, v, s2);
+        auto pixel = [&](const uint8_t *row, int x) {
+            if (P.pdt == 0) return u_to_float(row[x]);
+            if (P.pdt == 1) return u_to_float(reinterpret_cast<const uint16_t *>(row)[x]);
+            return reinterpret_cast<const float *>(row)[x];
+        };
+        if (pitch == W * bpp) {
+            constexpr int kBatch = 8;
+            for (int i0 = g.rank(); i0 < n; i0 += kBatch * g.size()) {
+                float v[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    const int i = i0 + k * g.size();
+                    if (i < n) v[k] = pixel(src, i);
                 }
-                img[i] = v;
+#pragma unroll
+                for (int k = 0; k < kBatch; k++) {
+                    const int i = i0 + k * g.size();
+                    if (i < n) img[i] = finish_pixel(v[k], i, P, off, gain);
+                }
+            }
+        } else {
+            const int rl = min(g.size(), 32);  // lanes along a row
+            const int lane = g.rank() & (rl - 1), wg = g.rank() / rl, nwg = g.size() / rl;
+            for (int y = wg; y < H; y += nwg) {
+                const uint8_t *row = src + (size_t)y * pitch;
+#pragma unroll 4
+                for (int x = lane; x < W; x += rl) {
+                    const int i = y * W + x;
+                    img[i] = finish_pixel(pixel(row, x), i, P, off, gain);
+                }
+            }
+        }
+        g.sync();
+        if (!chunked) {
+            for (int i = g.rank(); i < n; i += g.size()) {
+                const float v = img[i];
+                s += v;
+                s2 = fmaf(v, v, s2);
             }
         }
         if (chunked) {
-            g.sync();
             const float4 *img4 = reinterpret_cast<const float4 *>(img);
             for (int c = g.rank(); c < (n >> 2); c += g.size()) {
                 const float4 f = img4[c];
@@ -527,7 +585,7 @@ __device__ ComResult com_from_sums(const G &g, const float *img, int W, int H, f
     r.mean = (float)(s[0] * (double)invN);
     r.stdev = sqrtf((float)(s[1] * (double)invN - (double)(r.mean * r.mean)));
     const float thr = bgcorr * r.stdev;
-    float q0 = 0.0f, qx = 0.0f, qy = 0.0f;
+    double m[3] = {0.0, 0.0, 0.0};
     if (!(W & 3) && !(reinterpret_cast<uintptr_t>(img) & 15)) {
         // rows are whole float4 chunks: chunk c holds pixels 4c .. 4c+3 of one row, at column fx
         // and row fy; per chunk S = sum v', Sj = sum j v', so sum x v' = fx S + Sj
@@ -535,67 +593,66 @@ __device__ ComResult com_from_sums(const G &g, const float *img, int W, int H, f
         const float fW = (float)W, fdx = (float)(cstride % W), fdy = (float)(cstride / W);
         float fx = (float)((4 * g.rank()) % W), fy = (float)((4 * g.rank()) / W);
         const float4 *img4 = reinterpret_cast<const float4 *>(img);
-        for (int c = g.rank(); c < nc; c += stride) {
-            const float4 q = img4[c];
-            float a0, a1, a2, a3;
-            if (thr == 0.0f) {  // max(0, |d| - 0) is |d|
-                a0 = fabsf(q.x - r.mean);
-                a1 = fabsf(q.y - r.mean);
-                a2 = fabsf(q.z - r.mean);
-                a3 = fabsf(q.w - r.mean);
-            } else {
-                a0 = fmaxf(0.0f, fabsf(q.x - r.mean) - thr);
-                a1 = fmaxf(0.0f, fabsf(q.y - r.mean) - thr);
-                a2 = fmaxf(0.0f, fabsf(q.z - r.mean) - thr);
-                a3 = fmaxf(0.0f, fabsf(q.w - r.mean) - thr);
+        for (int c = g.rank(); c < nc;) {
+            float q0 = 0.0f, qx = 0.0f, qy = 0.0f;
+            for (const int end = min(nc, c + G::kFold / 4 * stride); c < end; c += stride) {
+                const float4 q = img4[c];
+                float a0, a1, a2, a3;
+                if (thr == 0.0f) {  // max(0, |d| - 0) is |d|
+                    a0 = fabsf(q.x - r.mean);
+                    a1 = fabsf(q.y - r.mean);
+                    a2 = fabsf(q.z - r.mean);
+                    a3 = fabsf(q.w - r.mean);
+                } else {
+                    a0 = fmaxf(0.0f, fabsf(q.x - r.mean) - thr);
+                    a1 = fmaxf(0.0f, fabsf(q.y - r.mean) - thr);
+                    a2 = fmaxf(0.0f, fabsf(q.z - r.mean) - thr);
+                    a3 = fmaxf(0.0f, fabsf(q.w - r.mean) - thr);
+                }
+                const float S = (a0 + a1) + (a2 + a3);
+                const float Sj = fmaf(3.0f, a3, fmaf(2.0f, a2, a1));
+                q0 += S;
+                qx += fmaf(fx, S, Sj);
+                qy = fmaf(fy, S, qy);
+                fx += fdx;
+                fy += fdy;
+                if (fx >= fW) {
+                    fx -= fW;
+                    fy += 1.0f;
+                }
             }
-            const float S = (a0 + a1) + (a2 + a3);
-            const float Sj = fmaf(3.0f, a3, fmaf(2.0f, a2, a1));
-            q0 += S;
-            qx += fmaf(fx, S, Sj);
-            qy = fmaf(fy, S, qy);
-            fx += fdx;
-            fy += fdy;
-            if (fx >= fW) {
-                fx -= fW;
-                fy += 1.0f;
-            }
+            m[0] += (double)q0;
+            m[1] += (double)qx;
+            m[2] += (double)qy;
         }
     } else {
         int x = g.rank() % W, y = g.rank() / W;
         float fx = (float)x, fy = (float)y;
-        for (int i = g.rank(); i < n; i += stride) {
-            const float v = fmaxf(0.0f, fabsf(img[i] - r.mean) - thr);
-            q0 += v;
-            qx += fx * v;
-            qy += fy * v;
-            x += dx;
-            fx += (float)dx;
-            fy += (float)dy;
-            if (x >= W) {
-                x -= W;
-                fx -= (float)W;
-                fy += 1.0f;
+        for (int i = g.rank(); i < n;) {
+            float q0 = 0.0f, qx = 0.0f, qy = 0.0f;
+            for (const int end = min(n, i + G::kFold * stride); i < end; i += stride) {
+                const float v = fmaxf(0.0f, fabsf(img[i] - r.mean) - thr);
+                q0 += v;
+                qx += fx * v;
+                qy += fy * v;
+                x += dx;
+                fx += (float)dx;
+                fy += (float)dy;
+                if (x >= W) {
+                    x -= W;
+                    fx -= (float)W;
+                    fy += 1.0f;
+                }
             }
+            m[0] += (double)q0;
+            m[1] += (double)qx;
+            m[2] += (double)qy;
         }
     }
-    double m[3] = {q0, qx, qy};
     g.sum(m);
     r.x = (float)(m[1] / m[0]);
     r.y = (float)(m[2] / m[0]);
     return r;
-}
-
-template <class G>
-__device__ ComResult compute_com(const G &g, const float *img, int W, int H, float bgcorr)
-{
-    float p0 = 0.0f, p1 = 0.0f;
-    for (int i = g.rank(); i < W * H; i += g.size()) {
-        const float v = img[i];
-        p0 += v;
-        p1 += v * v;
-    }
-    return com_from_sums(g, img, W, H, make_float2(p0, p1), bgcorr);
 }
 
 // Bilinear value at a sample whose truncated corner (ix, row) and fractions are known: row points

@@ -12,8 +12,14 @@ namespace qtrk {
 void plan_smem(TrackParams &P);
 // Raise the dynamic shared-memory limit of the kernels once per device.
 cudaError_t prepare_kernels(int device);
-// True when the Gaussian-only warp-per-ROI kernel serves P.
+// The Gaussian-only mode on ROIs of at most 32x32 pixels (gauss.cu, one warp per ROI): whether it
+// serves P, its launch, and its graph node (function, grid, block, shared memory).
 bool use_gauss_warp(const TrackParams &P);
+cudaError_t prepare_gauss_kernels();
+void gauss_warp_node(const TrackParams &P, int count, cudaKernelNodeParams &kp);
+cudaError_t launch_gauss_warp(const TrackParams &P, const uint8_t *pixels, int pitch, int64_t roi_stride,
+                              const int64_t *roi_offsets, const LocalizationJob *jobs, int count,
+                              LocalizationResult *results, cudaStream_t stream);
 
 // Localize `count` ROIs: ROI i starts at pixels + (roi_offsets ? roi_offsets[i] : i*roi_stride).
 // jobs may be null (job i = {frame=i}). One kernel launch.

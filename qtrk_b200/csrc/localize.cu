@@ -6,7 +6,6 @@
 //   first COM pass -> COM -> QI iterations -> radial profile -> Z-LUT match -> result. Pixels are
 //   read from HBM exactly once; everything after the load works on-chip.
 // localize_gauss_kernel: one CTA per ROI, COM -> 2D Gaussian MLE (-> Z) on a plain tile.
-// gauss_warp_kernel: one warp per small ROI (<= 32x32) for the Gaussian-only mode.
 // build_lut_kernel / finalize_lut_kernel: QueuedCPUTracker::BuildLUT / FinalizeLUT
 //   (cputrack/QueuedCPUTracker.cpp:580-659) with the accumulation on the device.
 // profile_kernel: ComputeRadialProfile (cputrack/utils.cpp:275-320) for one image.
@@ -232,34 +231,6 @@ __device__ float z_localize(const SmemView &s, const TrackParams &P, float mean,
     return s.misc[2];
 }
 
-__device__ __forceinline__ void read_job(const LocalizationJob *jobs, int i, uint32_t (&w)[6])
-{
-    if (jobs) {
-        const uint32_t *p = reinterpret_cast<const uint32_t *>(jobs) + (size_t)i * 6;
-#pragma unroll
-        for (int k = 0; k < 6; k++) w[k] = p[k];
-    } else {
-        w[0] = (uint32_t)i;
-#pragma unroll
-        for (int k = 1; k < 6; k++) w[k] = 0;
-    }
-}
-
-__device__ __forceinline__ void write_result(LocalizationResult *results, int i, const uint32_t (&job)[6], float x,
-                                             float y, float z, float gx, float gy, uint32_t err, float mean)
-{
-    uint32_t *o = reinterpret_cast<uint32_t *>(results) + (size_t)i * 13;
-#pragma unroll
-    for (int k = 0; k < 6; k++) o[k] = job[k];
-    o[6] = __float_as_uint(x);
-    o[7] = __float_as_uint(y);
-    o[8] = __float_as_uint(z);
-    o[9] = __float_as_uint(gx);
-    o[10] = __float_as_uint(gy);
-    o[11] = err;
-    o[12] = __float_as_uint(mean);
-}
-
 constexpr int kMinBlocks = 5;  // CTAs per SM the QI and Gaussian kernels are compiled for (<= 96 registers)
 
 constexpr uint32_t kStageWaitLimit = 1u << 22;  // mbarrier polls before a staged copy counts as lost
@@ -344,8 +315,8 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
     BlockGroup g{s.red};
     const int W = P.width, H = P.height;
-    load_roi(g, s.img, pixels + off, pitch, P, bead);
-    const ComResult com = compute_com(g, s.img, W, H, P.com_bgcorrection);
+    const float2 part = load_roi(g, s.img, pixels + off, pitch, P, bead);
+    const ComResult com = com_from_sums(g, s.img, W, H, part, P.com_bgcorrection);
     float comx = com.x, comy = com.y;
     if (isnan(comx) || isnan(comy)) {  // QueuedCPUTracker.cpp:294-295
         comx = (float)(W / 2);
@@ -369,46 +340,6 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
         z = z_localize(s, P, com.mean, x, y, bead, roi);
     }
     if (threadIdx.x == 0) write_result(results, roi, job, x, y, z, comx, comy, bhit ? 1u : 0u, com.mean);
-}
-
-// Gaussian-only mode for ROIs of at most 32x32 pixels: one warp per ROI, 8 ROIs per CTA. Three
-// CTAs per SM (80 registers, a few spilled) beat two without spills by 22-35 % on 16x16 ROIs.
-__global__ void __launch_bounds__(256, 3) gauss_warp_kernel(TrackParams P, const uint8_t *__restrict__ pixels, int pitch,
-                                                         int64_t roi_stride, const int64_t *__restrict__ roi_offsets,
-                                                         const LocalizationJob *__restrict__ jobs, int count,
-                                                         LocalizationResult *__restrict__ results)
-{
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int warp = threadIdx.x >> 5;
-    const int roi = blockIdx.x * 8 + warp;
-    if (roi >= count) return;  // whole warps exit together
-    const int W = P.width, H = P.height;
-    const int per_warp = ((W * H + 3 * (W + H) + 3) & ~3) * 4;
-    float *img = reinterpret_cast<float *>(smem + warp * per_warp);
-    float *col = img + W * H;
-    float *row = col + 3 * W;
-    uint32_t job[6];
-    read_job(jobs, roi, job);
-    const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
-    WarpGroup g;
-    load_roi(g, img, pixels + off, pitch, P, (int)job[2]);
-    const ComResult com = compute_com(g, img, W, H, P.com_bgcorrection);
-    float comx = com.x, comy = com.y;
-    if (isnan(comx) || isnan(comy)) {
-        comx = (float)(W / 2);
-        comy = (float)(H / 2);
-    }
-    float x = comx, y = comy, z = 0.0f;
-    if (P.mode & kLT_Gaussian5P) {
-        float p[5] = {x, y, com.mean * 0.5f * (float)(W * H), com.mean * 0.5f, P.g_sigma};
-        gauss5_mle(g, img, W, H, p, P.g_iterations, col, row);
-        x = p[0];
-        y = p[1];
-        z = p[4];
-    } else {
-        gauss4_mle(g, img, W, H, com.mean, x, y, P.g_iterations, P.g_sigma, col, row);
-    }
-    if ((threadIdx.x & 31) == 0) write_result(results, roi, job, x, y, z, comx, comy, 0u, com.mean);
 }
 
 // One bead of QueuedCPUTracker::BuildLUT (QueuedCPUTracker.cpp:582-645): ROI i of the stack is
@@ -519,12 +450,6 @@ void plan_smem(TrackParams &P)
     P.smem_bytes = P.sm_misc + 64;
 }
 
-int gauss_warp_smem(const TrackParams &P)
-{
-    const int W = P.width, H = P.height;
-    return 8 * ((W * H + 3 * (W + H) + 3) & ~3) * 4;
-}
-
 static bool g_attrs_set[64];
 
 cudaError_t prepare_kernels(int device)
@@ -541,14 +466,9 @@ cudaError_t prepare_kernels(int device)
         return e;
     if ((e = cudaFuncSetAttribute(build_lut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem))) return e;
     if ((e = cudaFuncSetAttribute(profile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem))) return e;
-    if ((e = cudaFuncSetAttribute(gauss_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem))) return e;
+    if ((e = prepare_gauss_kernels())) return e;
     g_attrs_set[device] = true;
     return cudaSuccess;
-}
-
-bool use_gauss_warp(const TrackParams &P)
-{
-    return (P.mode & kLT_Gaussian2D) && !(P.mode & (kLT_QI | kLT_LocalizeZ)) && P.width <= 32 && P.height <= 32;
 }
 
 cudaError_t launch_localize(const TrackParams &P, const uint8_t *pixels, int pitch, int64_t roi_stride,
@@ -558,10 +478,9 @@ cudaError_t launch_localize(const TrackParams &P, const uint8_t *pixels, int pit
     if (count <= 0) return cudaSuccess;
     if (use_com_kernel(P, pixels, pitch, roi_stride, roi_offsets))
         return launch_com(P, pixels, roi_stride, jobs, count, results, stream);
-    if (use_gauss_warp(P)) {
-        gauss_warp_kernel<<<(count + 7) / 8, 256, gauss_warp_smem(P), stream>>>(P, pixels, pitch, roi_stride,
-                                                                              roi_offsets, jobs, count, results);
-    } else if ((P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI)) {
+    if (use_gauss_warp(P))
+        return launch_gauss_warp(P, pixels, pitch, roi_stride, roi_offsets, jobs, count, results, stream);
+    if ((P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI)) {
         localize_gauss_kernel<<<count, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, roi_stride,
                                                                               roi_offsets, jobs, count, results);
     } else {
@@ -659,10 +578,7 @@ void localize_node(const TrackParams &P, int count, cudaKernelNodeParams &kp)
 {
     kp = cudaKernelNodeParams{};
     if (use_gauss_warp(P)) {
-        kp.func = reinterpret_cast<void *>(gauss_warp_kernel);
-        kp.gridDim = dim3((count + 7) / 8);
-        kp.blockDim = dim3(256);
-        kp.sharedMemBytes = gauss_warp_smem(P);
+        gauss_warp_node(P, count, kp);
     } else {
         kp.func = (P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI) ? reinterpret_cast<void *>(localize_gauss_kernel)
                                                                    : reinterpret_cast<void *>(localize_qi_kernel<false>);
