@@ -357,7 +357,8 @@ __global__ void __launch_bounds__(kAdjThreads) joint_refine_kernel(TrackParams P
 
 // Gaussian-MLE adjoint: Poisson NLL = sum mu - I ln mu of the 5-parameter integrated-Gaussian
 // model (the model gauss5_mle fits, erff per column/row, FP32 per pixel, FP64 sums) and its
-// gradient sum (1 - I/mu) dmu/dp for p = (x, y, I0, bg, sigma) = params[5 roi ..]. One block per ROI.
+// gradient sum (1 - I/mu) dmu/dp for p = (x, y, I0, bg, sigma) = params[5 roi ..]. One block per ROI;
+// windows of at most 32x32 pixels take gauss_nll_warp_kernel (gauss.cu).
 __global__ void __launch_bounds__(kAdjThreads) gauss_nll_grad_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
                                                                      int pitch, int64_t roi_stride, int count,
                                                                      const float *__restrict__ params,
@@ -433,6 +434,7 @@ cudaError_t launch_gauss_nll_grad(const TrackParams &P, const uint8_t *pixels, i
                                   const float *params, float *nll, float *grad, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
+    if (use_gauss_nll_warp(P)) return launch_gauss_nll_warp(P, pixels, pitch, roi_stride, count, params, nll, grad, stream);
     const int W = P.width, H = P.height;
     const int smem = (int)((((size_t)((W * H + 3) & ~3) + 3 * (W + H)) * 4 + 15) / 16 * 16) + 6 * 32 * 8;
     cudaError_t e = cudaFuncSetAttribute(gauss_nll_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

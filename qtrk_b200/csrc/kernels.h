@@ -21,6 +21,12 @@ cudaError_t launch_gauss_warp(const TrackParams &P, const uint8_t *pixels, int p
                               const int64_t *roi_offsets, const LocalizationJob *jobs, int count,
                               LocalizationResult *results, cudaStream_t stream);
 
+// The Gaussian likelihood gradient of windows of at most 32x32 pixels (gauss.cu); launch_gauss_nll_grad
+// chooses it by itself.
+bool use_gauss_nll_warp(const TrackParams &P);
+cudaError_t launch_gauss_nll_warp(const TrackParams &P, const uint8_t *pixels, int pitch, int64_t roi_stride, int count,
+                                  const float *params, float *nll, float *grad, cudaStream_t stream);
+
 // Localize `count` ROIs: ROI i starts at pixels + (roi_offsets ? roi_offsets[i] : i*roi_stride).
 // jobs may be null (job i = {frame=i}). One kernel launch.
 cudaError_t launch_localize(const TrackParams &P, const uint8_t *pixels, int pitch, int64_t roi_stride,

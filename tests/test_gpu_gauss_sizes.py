@@ -56,3 +56,33 @@ def test_gauss_window_sizes_match_fp64(port, w, h, params):
             if params == 5:
                 assert abs(r["pos"][i, 2] - want[4]) < 2e-5
         assert checked >= n - 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", SIZES + [(33, 20)])
+def test_gauss_nll_gradient_window_sizes_match_fp64(port, w, h):
+    """Likelihood and gradient at the same sizes (33 columns: the CTA form). FP32 residuals of a few 1e-7
+    relative, summed in FP64: 1e-6 of the likelihood and 1e-5 of each component's sum of magnitudes."""
+    import torch
+
+    n = 13
+    for dtype in (np.float32, np.uint16):
+        rois, sigma = spots(w, h, n, dtype, 7 * w + h)
+        rng = np.random.Generator(np.random.PCG64(w + h))
+        prm = np.stack([w / 2 + rng.uniform(-.5, .5, n), h / 2 + rng.uniform(-.5, .5, n), 10.0 * w * h * rng.uniform(.5, 1.5, n),
+                        rng.uniform(8, 12, n), sigma * rng.uniform(.9, 1.1, n)], 1).astype(np.float32)
+        px = torch.from_numpy(rois if dtype == np.float32 else rois.view(np.int16)).cuda()
+        p, nll, grad = torch.from_numpy(prm).cuda(), torch.empty(n, device="cuda"), torch.empty(n, 5, device="cuda")
+        s = abi.settings(width=w, height=h, gauss2D_sigma=sigma, qi_minradius=1, zlut_minradius=0.25)
+        b = rois.itemsize
+        with QTrkInstance(s) as t:
+            assert t.lib.QTrkB200GaussianNLLGradient(t.handle, px.data_ptr(), w * b, w * h * b, abi.NUMPY_PDT[rois.dtype], n,
+                                                     p.data_ptr(), nll.data_ptr(), grad.data_ptr(), None) == 0
+            torch.cuda.synchronize()
+        for i in range(n):
+            want, g = port.gauss_nll_grad(rois[i].astype(np.float64), prm[i].astype(np.float64))
+            assert abs(float(nll[i]) - want) < 1e-6 * max(abs(want), 10.0 * w * h)
+            # each residual f is off by a few 1e-7 of max(f, 1); the derivative's magnitudes sum to `scale`
+            for k in range(5):
+                scale = max(1.0, abs(prm[i, 2]) if k in (0, 1, 4) else float(w * h if k == 3 else 1.0))
+                assert abs(float(grad[i, k]) - g[k]) < 1e-5 * scale + 1e-5 * abs(g[k]), (i, k)
