@@ -83,68 +83,11 @@ struct LaneGroup {
     }
 };
 
-// Interpolate, utils.h:40-58: rx = (int)x (C truncation); the sample is outside when rx < 0,
-// ry < 0, rx+1 >= w or ry+1 >= h. Returns false when outside. Row y of the tile starts at
-// img + y * ts (ts >= w: the tile's row pitch in floats).
-// Without float->int conversions: truncation keeps a sample inside exactly when -1 < x < w-1,
-// and for those x, (int)x == floor(max(x, 0)), which a round-toward-zero add of 2^23 puts in
-// the low mantissa bits. The fraction x - rx is formed from the same exact float as the
+// Bilinear sampling follows Interpolate, utils.h:40-58: rx = (int)x (C truncation); the sample is outside when
+// rx < 0, ry < 0, rx+1 >= w or ry+1 >= h. No float->int conversions: truncation keeps a sample inside
+// exactly when -1 < x < w-1, and for those x, (int)x == floor(max(x, 0)), which a round-toward-zero add
+// of 2^23 puts in the low mantissa bits. The fraction x - rx is formed from the same exact float as the
 // reference's x - (float)rx, so the interpolated value is unchanged.
-__device__ __forceinline__ bool bilinear(const float *img, int w, int h, int ts, float x, float y, float &v)
-{
-    if (!(x > -1.0f && x < (float)(w - 1) && y > -1.0f && y < (float)(h - 1))) return false;
-    const float kMagic = 8388608.0f;  // 2^23
-    const float tx = __fadd_rz(fmaxf(x, 0.0f), kMagic), ty = __fadd_rz(fmaxf(y, 0.0f), kMagic);
-    const int rx = __float_as_int(tx) - 0x4B000000, ry = __float_as_int(ty) - 0x4B000000;
-    const float *p = img + ry * ts + rx;
-    const float v00 = p[0], v10 = p[1], v01 = p[ts], v11 = p[ts + 1];
-    const float fx = x - (tx - kMagic), fy = y - (ty - kMagic);
-    const float v0 = v00 + (v10 - v00) * fx;
-    const float v1 = v01 + (v11 - v01) * fx;
-    v = v0 + (v1 - v0) * fy;
-    return true;
-}
-
-// bilinear() for a sample known to lie strictly inside (0 < x < w-1, 0 < y < h-1): the same
-// arithmetic without the range test. Callers prove the range for a whole bin at once.
-__device__ __forceinline__ float bilinear_inside(const float *img, int ts, float x, float y)
-{
-    const float kMagic = 8388608.0f;
-    const float tx = __fadd_rz(x, kMagic), ty = __fadd_rz(y, kMagic);
-    const float *p = img + ((__float_as_int(ty) - 0x4B000000) * ts + (__float_as_int(tx) - 0x4B000000));
-    const float v00 = p[0], v10 = p[1], v01 = p[ts], v11 = p[ts + 1];
-    const float fx = x - (tx - kMagic), fy = y - (ty - kMagic);
-    const float v0 = v00 + (v10 - v00) * fx;
-    const float v1 = v01 + (v11 - v01) * fx;
-    return v0 + (v1 - v0) * fy;
-}
-
-// Two bilinear samples at once with the packed FP32x2 operations of sm_100 (each component
-// rounds as the scalar operation does): cells at p and q, fractions fx = (fx_p, fx_q) and
-// fy = (fy_p, fy_q). Same arithmetic as lerp_cell, one instruction per pair of samples; the
-// differences v10 - v00 are fma(v00, -1, v10), exact before their one rounding.
-__device__ __forceinline__ float2 lerp_cell2(const float *p, const float *q, int ts, float2 fx, float2 fy)
-{
-    const float2 m1 = make_float2(-1.0f, -1.0f);
-    const float2 v00 = make_float2(p[0], q[0]), v10 = make_float2(p[1], q[1]);
-    const float2 v01 = make_float2(p[ts], q[ts]), v11 = make_float2(p[ts + 1], q[ts + 1]);
-    const float2 v0 = __ffma2_rn(__ffma2_rn(v00, m1, v10), fx, v00);
-    const float2 v1 = __ffma2_rn(__ffma2_rn(v01, m1, v11), fx, v01);
-    return __ffma2_rn(__ffma2_rn(v0, m1, v1), fy, v0);
-}
-
-// bilinear_inside for two samples at (X.x, Y.x) and (X.y, Y.y) with packed FP32x2 arithmetic
-// (each component rounded as bilinear_inside rounds it).
-__device__ __forceinline__ float2 bilinear_inside2(const float *img, int ts, float2 X, float2 Y)
-{
-    const float2 K = make_float2(8388608.0f, 8388608.0f), nK = make_float2(-8388608.0f, -8388608.0f);
-    const float2 m1 = make_float2(-1.0f, -1.0f);
-    const float2 TX = __fadd2_rz(X, K), TY = __fadd2_rz(Y, K);
-    const float2 FX = __ffma2_rn(__fadd2_rn(TX, nK), m1, X), FY = __ffma2_rn(__fadd2_rn(TY, nK), m1, Y);
-    const float *p = img + ((__float_as_int(TY.x) - 0x4B000000) * ts + (__float_as_int(TX.x) - 0x4B000000));
-    const float *q = img + ((__float_as_int(TY.y) - 0x4B000000) * ts + (__float_as_int(TX.y) - 0x4B000000));
-    return lerp_cell2(p, q, ts, FX, FY);
-}
 
 // True when every point cx + a*r, cy + b*r with |a|, |b| <= 1 (any sample of a circle of radius
 // r around (cx, cy)) lies strictly inside (0, w-1) x (0, h-1), rounding of the sample
@@ -163,12 +106,13 @@ __device__ __forceinline__ bool check_boundaries(float cx, float cy, float radiu
 
 // LsqSqQuadFit + ComputeMaxInterp<T,7>::Compute (LsqQuadraticFit.h:8-176) in FP64, with the eight
 // weighted sums formed by lanes 0..6 of one warp (all 32 lanes call; every lane returns the result).
-// `at(i)` returns element i of the length-`len` array; iMax is the first index of the maximum;
+// `at(i)` returns element i of the length-`len` array, iMax is the first index of the maximum;
 // the weights are indexed from 0 even when the window is clipped at the array start, as in the
 // reference. maxPos = iMax - b/(2a) with a = A/d, b = B/d, so the
 // determinant d cancels and one division remains; |a| < 1e-9 is tested as |A| < 1e-9 |d|.
-template <typename Get>
-__device__ inline double max_interp7_warp(Get at, int len, int iMax, const float (&wts)[7])
+// y is element max(iMax - 3, 0) + lane of the array (read by lanes below the window's length). Not inlined:
+// a rare path, and the localization kernel's time depends on how much of it stays in the instruction cache.
+static __device__ __noinline__ double max_interp7_clipped(double y, int len, int iMax, const float (&wts)[7])
 {
     const int lane = threadIdx.x & 31;
     const int startPos = max(iMax - 3, 0);
@@ -177,7 +121,7 @@ __device__ inline double max_interp7_warp(Get at, int len, int iMax, const float
     if (np < 3) return (double)iMax;
     double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (lane < np) {
-        const double x = (double)(startPos + lane - iMax), y = (double)at(startPos + lane), wt = (double)wts[lane];
+        const double x = (double)(startPos + lane - iMax), wt = (double)wts[lane];
         const double sq = x * x;
         t[0] = x * wt;        // Sx
         t[1] = y * wt;        // Sy
@@ -200,6 +144,13 @@ __device__ inline double max_interp7_warp(Get at, int len, int iMax, const float
     const double B = Sx4 * (Sxy * Sw - Sy * Sx) - Sx3 * (Sx2y * Sw - Sy * Sx2) + Sx2 * (Sx2y * Sx - Sxy * Sx2);
     if (fabs(A) < 1e-9 * fabs(d)) return (double)iMax;
     return (double)iMax - B / (2 * A);
+}
+
+template <typename Get>
+__device__ __forceinline__ double max_interp7_warp(Get at, int len, int iMax, const float (&wts)[7])
+{
+    const int i = max(iMax - 3, 0) + (threadIdx.x & 31);
+    return max_interp7_clipped(i < min(iMax + 4, len) ? (double)at(i) : 0.0, len, iMax, wts);
 }
 
 // The same fit for the common case, a window iMax-3 .. iMax+3 inside the array with weights
@@ -304,13 +255,13 @@ __device__ __forceinline__ void write_result(LocalizationResult *results, int i,
 // placing it in the mantissa of 2^23 and subtracting 2^23.
 __device__ __forceinline__ float u_to_float(uint32_t u) { return __uint_as_float(0x4B000000u | u) - 8388608.0f; }
 
-__device__ __forceinline__ float finish_pixel(float v, int i, const TrackParams &P, const float *off,
-                                              const float *gain)
+__device__ __forceinline__ float finish_pixel(float v, int i, int mode, float off_factor, float gain_factor,
+                                              const float *off, const float *gain)
 {
-    if ((P.mode & kLT_ClearFirstFourPixels) && i < 4) v = 0.0f;
-    if (off && !gain) v = v + off[i] * P.offset_factor;
-    if (gain && !off) v = v * gain[i] * P.gain_factor;
-    if (gain && off) v = (v + off[i] * P.offset_factor) * gain[i] * P.gain_factor;
+    if ((mode & kLT_ClearFirstFourPixels) && i < 4) v = 0.0f;
+    if (off && !gain) v = v + off[i] * off_factor;
+    if (gain && !off) v = v * gain[i] * gain_factor;
+    if (gain && off) v = (v + off[i] * off_factor) * gain[i] * gain_factor;
     return v;
 }
 
@@ -341,10 +292,10 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
         float4 *dst = reinterpret_cast<float4 *>(img);
         auto finish4 = [&](float4 f, int c) {
             if (!plain) {
-                f.x = finish_pixel(f.x, 4 * c, P, off, gain);
-                f.y = finish_pixel(f.y, 4 * c + 1, P, off, gain);
-                f.z = finish_pixel(f.z, 4 * c + 2, P, off, gain);
-                f.w = finish_pixel(f.w, 4 * c + 3, P, off, gain);
+                f.x = finish_pixel(f.x, 4 * c, P.mode, P.offset_factor, P.gain_factor, off, gain);
+                f.y = finish_pixel(f.y, 4 * c + 1, P.mode, P.offset_factor, P.gain_factor, off, gain);
+                f.z = finish_pixel(f.z, 4 * c + 2, P.mode, P.offset_factor, P.gain_factor, off, gain);
+                f.w = finish_pixel(f.w, 4 * c + 3, P.mode, P.offset_factor, P.gain_factor, off, gain);
             }
             s += f.x;
             s2 = fmaf(f.x, f.x, s2);
@@ -438,7 +389,7 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
 #pragma unroll
                 for (int k = 0; k < kBatch; k++) {
                     const int i = i0 + k * g.size();
-                    if (i < n) img[i] = finish_pixel(v[k], i, P, off, gain);
+                    if (i < n) img[i] = finish_pixel(v[k], i, P.mode, P.offset_factor, P.gain_factor, off, gain);
                 }
             }
         } else {
@@ -449,7 +400,7 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
 #pragma unroll 4
                 for (int x = lane; x < W; x += rl) {
                     const int i = y * W + x;
-                    img[i] = finish_pixel(pixel(row, x), i, P, off, gain);
+                    img[i] = finish_pixel(pixel(row, x), i, P.mode, P.offset_factor, P.gain_factor, off, gain);
                 }
             }
         }
@@ -474,84 +425,6 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
                 s += f.w;
                 s2 = fmaf(f.w, f.w, s2);
             }
-        }
-    }
-    g.sync();
-    return make_float2(s, s2);
-}
-
-// load_roi for a ROI whose raw bytes (n = W*H pixels, u8/u16/f32, rows back to back) were brought
-// into shared memory by a bulk copy to img + (4 - bpp) n bytes, the end of the float tile. The
-// conversion runs in place in batches of kBatch chunks of four pixels per thread: a batch's raw
-// chunks are read into registers, a barrier passes, and the batch's float chunks are written.
-// Float chunk c (bytes 16c .. 16c+15) overlaps only raw chunks with index <= c, which the batch or
-// an earlier one has already read, so a batch never overwrites raw bytes a later batch needs. The
-// per-pixel steps and the returned partial sums are load_roi's. Requires n a multiple of 4. All
-// threads call; the tile is complete at return.
-template <class G>
-__device__ inline float2 convert_staged(const G &g, float *img, const TrackParams &P, int bead)
-{
-    const int W = P.width, H = P.height, n = W * H, nc = n >> 2;
-    const int bpp = P.pdt == 0 ? 1 : (P.pdt == 1 ? 2 : 4);
-    const uint8_t *raw = reinterpret_cast<const uint8_t *>(img) + (size_t)(4 - bpp) * n;
-    const float *off = nullptr, *gain = nullptr;
-    if (bead >= 0 && bead < P.calib_count) {
-        if (P.calib_offset) off = P.calib_offset + (size_t)bead * n;
-        if (P.calib_gain) gain = P.calib_gain + (size_t)bead * n;
-    }
-    const bool plain = !off && !gain && !(P.mode & kLT_ClearFirstFourPixels);
-    float4 *dst = reinterpret_cast<float4 *>(img);
-    float s = 0.0f, s2 = 0.0f;
-    constexpr int kBatch = 8;
-    // every thread runs the same number of batches (the loop holds a barrier)
-    for (int b0 = 0; b0 < nc; b0 += kBatch * g.size()) {
-        const int c0 = b0 + g.rank();
-        uint4 q[kBatch];
-#pragma unroll
-        for (int k = 0; k < kBatch; k++) {
-            const int c = c0 + k * g.size();
-            if (c < nc) {
-                if (P.pdt == 0) {
-                    q[k].x = reinterpret_cast<const uint32_t *>(raw)[c];
-                } else if (P.pdt == 1) {
-                    const uint2 v = reinterpret_cast<const uint2 *>(raw)[c];
-                    q[k].x = v.x;
-                    q[k].y = v.y;
-                } else {
-                    q[k] = reinterpret_cast<const uint4 *>(raw)[c];
-                }
-            }
-        }
-        g.sync();
-#pragma unroll
-        for (int k = 0; k < kBatch; k++) {
-            const int c = c0 + k * g.size();
-            if (c >= nc) continue;
-            float4 f;
-            if (P.pdt == 0)
-                f = make_float4(u_to_float(q[k].x & 0xffu), u_to_float((q[k].x >> 8) & 0xffu),
-                                u_to_float((q[k].x >> 16) & 0xffu), u_to_float(q[k].x >> 24));
-            else if (P.pdt == 1)
-                f = make_float4(u_to_float(q[k].x & 0xffffu), u_to_float(q[k].x >> 16), u_to_float(q[k].y & 0xffffu),
-                                u_to_float(q[k].y >> 16));
-            else
-                f = make_float4(__uint_as_float(q[k].x), __uint_as_float(q[k].y), __uint_as_float(q[k].z),
-                                __uint_as_float(q[k].w));
-            if (!plain) {
-                f.x = finish_pixel(f.x, 4 * c, P, off, gain);
-                f.y = finish_pixel(f.y, 4 * c + 1, P, off, gain);
-                f.z = finish_pixel(f.z, 4 * c + 2, P, off, gain);
-                f.w = finish_pixel(f.w, 4 * c + 3, P, off, gain);
-            }
-            s += f.x;
-            s2 = fmaf(f.x, f.x, s2);
-            s += f.y;
-            s2 = fmaf(f.y, f.y, s2);
-            s += f.z;
-            s2 = fmaf(f.z, f.z, s2);
-            s += f.w;
-            s2 = fmaf(f.w, f.w, s2);
-            dst[c] = f;
         }
     }
     g.sync();
@@ -655,196 +528,6 @@ __device__ ComResult com_from_sums(const G &g, const float *img, int W, int H, f
     return r;
 }
 
-// Bilinear value at a sample whose truncated corner (ix, row) and fractions are known: row points
-// at the tile row of the upper corner pixels. Arithmetic of bilinear_inside.
-__device__ __forceinline__ float lerp_cell(const float *row, int ts, int ix, float fx, float fy)
-{
-    const float *p = row + ix;
-    const float v00 = p[0], v10 = p[1], v01 = p[ts], v11 = p[ts + 1];
-    const float v0 = v00 + (v10 - v00) * fx;
-    const float v1 = v01 + (v11 - v01) * fx;
-    return v0 + (v1 - v0) * fy;
-}
-
-// CPUTracker::ComputeQuadrantProfile (cpu_tracker.cpp:631-677) for all four quadrants at once,
-// written as the FFT input of the QI autoconvolution. The four quadrants sample the same
-// table direction d at radius r with mirrored signs (x = cx +- d.x r, y = cy +- d.y r), so one
-// thread takes one radius and a strided subset of the directions and produces all four samples
-// of each: the products d.x r, d.y r, the truncations and fractions of the two x and two y
-// coordinates are shared by four samples. Coordinates are formed as the reference forms them
-// (d.x r rounded, then added to the centre). The table holds each direction as (d.x, d.x, d.y, d.y)
-// so that on the fast path x = (cx, cx) + (d.x, d.x) * (r, -r) gives (x+, x-) in one packed
-// multiply and one packed add; the diagonal quadrants q0 (+, +) and q2 (-, -) then share
-// fractions (fx+, fx-), (fy+, fy-) and are sampled as one pair, q3 (+, -) and q1 (-, +) as another. Layout: S = blockDim/nr direction subsets
-// (directions sub, sub + S, ...); a warp holds R = 32/A radii x A = min(S, 4) adjacent subsets,
-// so its gathers fall into a small patch. Per quadrant and radius the bin value
-// is the mean of the in-bounds samples (the image mean when fewer than 4), times the radial
-// weight; the subsets' partial sums meet through warp shuffles (and `part`, 2 KB of shared
-// memory, when S > A). The thread of subset 0 writes the X and Y concatenations
-// (cpu_tracker.cpp:327-343; X = [(q1+q2) reversed | q0+q3], Y = [(q2+q3) reversed | q0+q1]) as
-// one complex value z = X + iY per position, in bit-reversed order (log2L = log2(2 nr)) or in
-// natural order when log2L < 0. All threads call; a barrier must follow before A is read.
-__device__ __forceinline__ void qi_profiles_sym(const float *img, int W, int H, int ts, float cx, float cy, float mean, int nr,
-                                       int nang, float inv_nang, int stride, float minr, float rstep,
-                                       const float4 *dirs, const float *rweights, float4 *part, float2 *A, int log2L)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // nr and blockDim are powers of two (QTrkComputedConfig::Update rounds qi_radialsteps,
-    // QueuedTracker.cpp:20), so the layout is all shifts: S = 2^lS subsets, Aw = 2^lA of them per
-    // warp, R = 2^lR radii per warp, nwr = 2^lw warps along the radius, nsb subset blocks
-    const int lnr = ilog2_pow2(nr), lbd = ilog2_pow2(blockDim.x);
-    const int lS = lnr >= lbd ? 0 : lbd - lnr, lA = lS < 2 ? lS : 2, lR = 5 - lA;
-    const int lw = lnr >= lR ? lnr - lR : 0;
-    const int S = 1 << lS, Aw = 1 << lA, nwr = 1 << lw, nsb = 1 << (lS - lA);
-    const float kMagic = 8388608.0f;
-    for (int wi = warp; wi < nwr * nsb; wi += nw) {
-        const int rb = wi & (nwr - 1), sb = wi >> lw;
-        const int i = (rb << lR) + (lane >> lA), sub = (sb << lA) + (lane & (Aw - 1));
-        float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        int cnt[4] = {0, 0, 0, 0};
-        const float r = __fadd_rn(minr, __fmul_rn(rstep, (float)i));
-        // One path per warp: when any lane's circle may leave the image, the whole warp takes the
-        // checked body (a warp running both bodies one after the other would hold up the CTA's
-        // other warps at the next barrier).
-        const bool fast = __all_sync(0xffffffffu, i >= nr || circle_inside(cx, cy, fabsf(r), W, H));
-        if (i < nr) {
-            if (fast) {
-                const float2 rr = make_float2(r, -r), cxx = make_float2(cx, cx), cyy = make_float2(cy, cy);
-                const float2 K = make_float2(kMagic, kMagic), nK = make_float2(-kMagic, -kMagic);
-                const float2 m1 = make_float2(-1.0f, -1.0f);
-                float2 s02 = make_float2(0.0f, 0.0f), s31 = make_float2(0.0f, 0.0f);
-                for (int a = sub; a < nang; a += S) {
-                    const float4 d = dirs[stride * a];
-                    const float2 X = __fadd2_rn(cxx, __fmul2_rn(make_float2(d.x, d.y), rr));  // (x+, x-)
-                    const float2 Y = __fadd2_rn(cyy, __fmul2_rn(make_float2(d.z, d.w), rr));  // (y+, y-)
-                    const float2 TX = __fadd2_rz(X, K), TY = __fadd2_rz(Y, K);
-                    const float2 FX = __ffma2_rn(__fadd2_rn(TX, nK), m1, X);  // X - trunc(X)
-                    const float2 FY = __ffma2_rn(__fadd2_rn(TY, nK), m1, Y);
-                    const int ixp = __float_as_int(TX.x) - 0x4B000000, ixm = __float_as_int(TX.y) - 0x4B000000;
-                    const float *rowp = img + (__float_as_int(TY.x) - 0x4B000000) * ts;
-                    const float *rowm = img + (__float_as_int(TY.y) - 0x4B000000) * ts;
-                    s02 = __fadd2_rn(s02, lerp_cell2(rowp + ixp, rowm + ixm, ts, FX, FY));
-                    s31 = __fadd2_rn(s31, lerp_cell2(rowm + ixp, rowp + ixm, ts, FX, make_float2(FY.y, FY.x)));
-                }
-                sm[0] = s02.x;
-                sm[1] = s31.y;
-                sm[2] = s02.y;
-                sm[3] = s31.x;
-                const int c = sub < nang ? (nang - sub + S - 1) >> lS : 0;
-                cnt[0] = cnt[1] = cnt[2] = cnt[3] = c;
-            } else {
-                // bilinear()'s rule per coordinate: a sample is inside when -1 < x < W-1 and
-                // -1 < y < H-1, and its cell starts at the truncation of max(x, 0)
-                const float xhi = (float)(W - 1), yhi = (float)(H - 1);
-                for (int a = sub; a < nang; a += S) {
-                    const float4 d = dirs[stride * a];
-                    const float dx = __fmul_rn(d.x, r), dy = __fmul_rn(d.z, r);
-                    const float xp = __fadd_rn(cx, dx), xm = __fadd_rn(cx, -dx);
-                    const float yp = __fadd_rn(cy, dy), ym = __fadd_rn(cy, -dy);
-                    const bool vxp = xp > -1.0f && xp < xhi, vxm = xm > -1.0f && xm < xhi;
-                    const bool vyp = yp > -1.0f && yp < yhi, vym = ym > -1.0f && ym < yhi;
-                    const float txp = __fadd_rz(fmaxf(xp, 0.0f), kMagic), txm = __fadd_rz(fmaxf(xm, 0.0f), kMagic);
-                    const float typ = __fadd_rz(fmaxf(yp, 0.0f), kMagic), tym = __fadd_rz(fmaxf(ym, 0.0f), kMagic);
-                    const float fxp = xp - (txp - kMagic), fxm = xm - (txm - kMagic);
-                    const float fyp = yp - (typ - kMagic), fym = ym - (tym - kMagic);
-                    const int ixp = __float_as_int(txp) - 0x4B000000, ixm = __float_as_int(txm) - 0x4B000000;
-                    const float *rowp = img + (__float_as_int(typ) - 0x4B000000) * ts;
-                    const float *rowm = img + (__float_as_int(tym) - 0x4B000000) * ts;
-                    if (vxp && vyp) {
-                        sm[0] += lerp_cell(rowp, ts, ixp, fxp, fyp);
-                        cnt[0]++;
-                    }
-                    if (vxm && vyp) {
-                        sm[1] += lerp_cell(rowp, ts, ixm, fxm, fyp);
-                        cnt[1]++;
-                    }
-                    if (vxm && vym) {
-                        sm[2] += lerp_cell(rowm, ts, ixm, fxm, fym);
-                        cnt[2]++;
-                    }
-                    if (vxp && vym) {
-                        sm[3] += lerp_cell(rowm, ts, ixp, fxp, fym);
-                        cnt[3]++;
-                    }
-                }
-            }
-        }
-        // subsets of one radius: lanes that differ in their low log2(Aw) bits (on the fast path
-        // every count is nang: only the sums travel)
-        for (int o = 1; o < Aw; o <<= 1)
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                sm[q] += __shfl_xor_sync(0xffffffffu, sm[q], o);
-                if (!fast || nsb > 1) cnt[q] += __shfl_xor_sync(0xffffffffu, cnt[q], o);
-            }
-        if (nsb > 1) {  // subsets spread over warps (nr < blockDim/4): meet in shared memory
-            if ((lane & (Aw - 1)) == 0 && i < nr) {
-                part[2 * (sb * nr + i)] = make_float4(sm[0], sm[1], sm[2], sm[3]);
-                part[2 * (sb * nr + i) + 1] = make_float4(__int_as_float(cnt[0]), __int_as_float(cnt[1]),
-                                                          __int_as_float(cnt[2]), __int_as_float(cnt[3]));
-            }
-            continue;
-        }
-        float v[4];
-        if ((lane & (Aw - 1)) == 0 && i < nr) {
-            const float rw = rweights ? rweights[i] : 1.0f;
-            if (fast) {  // nang >= 4 in-bounds samples per bin: the mean, as sum * (1 / nang)
-#pragma unroll
-                for (int k = 0; k < 4; k++) v[k] = rweights ? (sm[k] * inv_nang) * rw : sm[k] * inv_nang;
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    v[k] = cnt[k] >= 4 ? sm[k] / (float)cnt[k] : mean;
-                    if (rweights) v[k] *= rw;
-                }
-            }
-        }
-        if ((lane & (Aw - 1)) == 0 && i < nr) {
-            const int n0 = nr - 1 - i, n1 = nr + i;
-            A[log2L >= 0 ? (int)bitrev(n0, log2L) : n0] = make_float2(v[1] + v[2], v[2] + v[3]);
-            A[log2L >= 0 ? (int)bitrev(n1, log2L) : n1] = make_float2(v[0] + v[3], v[0] + v[1]);
-        }
-    }
-    if (nsb > 1) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-            float sm[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            int cnt[4] = {0, 0, 0, 0};
-            for (int b = 0; b < nsb; b++) {
-                const float4 p = part[2 * (b * nr + i)], c = part[2 * (b * nr + i) + 1];
-                sm[0] += p.x;
-                sm[1] += p.y;
-                sm[2] += p.z;
-                sm[3] += p.w;
-                cnt[0] += __float_as_int(c.x);
-                cnt[1] += __float_as_int(c.y);
-                cnt[2] += __float_as_int(c.z);
-                cnt[3] += __float_as_int(c.w);
-            }
-            float v[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                v[q] = cnt[q] >= 4 ? sm[q] / (float)cnt[q] : mean;
-                if (rweights) v[q] *= rweights[i];
-            }
-            const int n0 = nr - 1 - i, n1 = nr + i;
-            A[log2L >= 0 ? (int)bitrev(n0, log2L) : n0] = make_float2(v[1] + v[2], v[2] + v[3]);
-            A[log2L >= 0 ? (int)bitrev(n1, log2L) : n1] = make_float2(v[0] + v[3], v[0] + v[1]);
-        }
-    }
-}
-
-// Lanes per radial-profile bin: the largest power of two with nbins*lanes <= threads, at least 4
-// (more than one pass over the bins when the CTA is small: with 128 threads and 64 bins, 4 lanes in
-// two passes ran 0.993 ms per 10,000 100x100 ROIs against 1.007 ms for 2 lanes in one), at most 32.
-__device__ __forceinline__ int lanes_per_bin(int nbins)
-{
-    int t = blockDim.x / nbins;
-    if (t < 4) t = 4;
-    if (t > 32) t = 32;
-    return 1 << (31 - __clz(t));
-}
-
 // Radix-2 decimation-in-time FFT of length L (power of two, input in bit-reversed order),
 // executed by one warp over shared memory. tw[k] = e^{-2 pi i k / L}, k < L/2.
 // Stage s pairs (i, i + 2^(s-1)) with twiddle tw[(i mod 2^(s-1)) * (L >> s)]. Two consecutive
@@ -926,163 +609,266 @@ __device__ inline void qi_autoconv_fft_filled(int nr, float2 *A, float2 *ac, con
 }
 
 
-// Same quantity by direct summation (any L; used when 2nr is not a power of two), A already
-// holding the packed profile in natural order and a barrier passed. All threads.
-__device__ inline void qi_autoconv_direct_filled(int nr, const float2 *A, float2 *ac)
+// The same correlation for L = 32 E (E = 1, 2, 4, 8 or 16), held in the registers of one warp: lane l has the
+// elements l + 32 e. The transform over e runs inside the lane, the 32-point transforms over the lanes by
+// shuffles (decimation in frequency forward, in time back, so no reordering pass lies between them:
+// lane l, slot e holds frequency bitrev(e) + E bitrev(l)). A holds the packed profile in natural order. The
+// passes through shared memory above load four elements and three twiddles per butterfly group and wait at a
+// warp barrier after each: with the fit, 3.8 k cycles for one update of 2 nr = 128 points alone on an SM, against
+// 1.5 k here (the instructions cached).
+__device__ __forceinline__ constexpr int bitrev_c(int v, int bits)
 {
-    const int L = 2 * nr;
-    for (int n = threadIdx.x; n < L; n += blockDim.x) {
-        float sx = 0.0f, sy = 0.0f;
-        for (int m = 0; m < L; m++) {
-            int idx = n + m;
-            if (idx >= L) idx -= L;
-            const float2 a = A[idx], b = A[L - 1 - m];
-            sx += a.x * b.x;
-            sy += a.y * b.y;
-        }
-        ac[n] = make_float2(L * sx, L * sy);
-    }
-    __syncthreads();
+    int r = 0;
+    for (int i = 0; i < bits; i++) r |= ((v >> i) & 1) << (bits - 1 - i);
+    return r;
 }
 
-// -------------------------------------------------------------------------------------
-// ComputeRadialProfile, utils.cpp:275-320: for each bin, the mean of the in-bounds
-// bilinear samples on the full circle (FP64 sum), or `mean` when no more than 4 samples
-// are in bounds; then NormalizeRadialProfile (utils.cpp:230-261) when asked.
-// -------------------------------------------------------------------------------------
-__device__ __forceinline__ void radial_profile(const float *img, int W, int H, int ts, float cx, float cy, float mean, int nb, int nang,
-                               float minr, float rstep, const float4 *dirs, float *prof, bool normalize,
-                               double *red)
+// z * e^{-2 pi i J / N} (or its conjugate) for compile-time J, N with N <= 16.
+template <int N, int J>
+__device__ __forceinline__ float2 cmul_root(float2 z, bool conj)
 {
-    // dirs[j] = (d_j.x, d_{j+h}.x, d_j.y, d_{j+h}.y) for j < h = nang/2, and d_{nang-1} alone in
-    // dirs[h] when nang is odd: each lane takes pairs j = sub, sub + tpb, ... (two samples per
-    // step, packed FP32x2) and lane 0 of each bin the unpaired direction.
-    const int tpb = lanes_per_bin(nb), ltpb = ilog2_pow2(tpb);
-    const int total = nb * tpb, h = nang >> 1;
-    const bool odd = (nang & 1) != 0;
-    for (int base = 0; base < total; base += blockDim.x) {
-        const int t = base + threadIdx.x;
-        const int bin = t >> ltpb, sub = t & (tpb - 1);
-        double sum = 0.0;
-        int cnt = 0;
-        const float r = minr + rstep * (float)bin;
-        // one path per warp (see qi_profiles_sym)
-        const bool inside = __all_sync(0xffffffffu, bin >= nb || circle_inside(cx, cy, fabsf(r), W, H));
-        if (bin < nb && inside) {
-            // Whole groups of 4 pairs (8 samples) are summed in FP32 and folded into an FP64
-            // total (the reference adds every sample in FP64; 8-sample FP32 groups stay within
-            // ~1e-7 of it), then the remaining pairs, then the unpaired direction.
-            const float2 rr = make_float2(r, r), cxx = make_float2(cx, cx), cyy = make_float2(cy, cy);
-            const int np = sub < h ? (h - sub + tpb - 1) >> ltpb : 0;
-            const float4 *dl = dirs + sub;
-            int k = 0;
-            for (; k + 4 <= np; k += 4) {
-                float2 part = make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const float4 d = dl[(k + u) << ltpb];
-                    part = __fadd2_rn(part, bilinear_inside2(img, ts, __ffma2_rn(make_float2(d.x, d.y), rr, cxx),
-                                                             __ffma2_rn(make_float2(d.z, d.w), rr, cyy)));
-                }
-                sum += (double)(part.x + part.y);
-            }
-            if (k < np) {
-                float2 part = make_float2(0.0f, 0.0f);
-                for (; k < np; k++) {
-                    const float4 d = dl[k << ltpb];
-                    part = __fadd2_rn(part, bilinear_inside2(img, ts, __ffma2_rn(make_float2(d.x, d.y), rr, cxx),
-                                                             __ffma2_rn(make_float2(d.z, d.w), rr, cyy)));
-                }
-                sum += (double)(part.x + part.y);
-            }
-            cnt = 2 * np;
-            if (odd && sub == 0) {
-                const float4 d = dirs[h];
-                sum += (double)bilinear_inside(img, ts, cx + d.x * r, cy + d.z * r);
-                cnt++;
-            }
-        } else if (bin < nb) {
-            // every sample checked; FP32 partials of up to 8 samples folded into FP64
-            for (int j0 = sub; j0 < h; j0 += 4 * tpb) {
-                float part = 0.0f;
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int j = j0 + u * tpb;
-                    if (j >= h) break;
-                    const float4 d = dirs[j];
-                    float v;
-                    if (bilinear(img, W, H, ts, cx + d.x * r, cy + d.z * r, v)) {
-                        part += v;
-                        cnt++;
-                    }
-                    if (bilinear(img, W, H, ts, cx + d.y * r, cy + d.w * r, v)) {
-                        part += v;
-                        cnt++;
-                    }
-                }
-                sum += (double)part;
-            }
-            if (odd && sub == 0) {
-                const float4 d = dirs[h];
-                float v;
-                if (bilinear(img, W, H, ts, cx + d.x * r, cy + d.z * r, v)) {
-                    sum += (double)v;
-                    cnt++;
-                }
-            }
-        }
-        for (int o = tpb >> 1; o > 0; o >>= 1) {
-            sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        }
-        if (bin < nb && sub == 0) prof[bin] = cnt > 4 ? (float)(sum / cnt) : mean;
-    }
-    __syncthreads();
-    if (normalize && threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        double s = 0;
-        for (int i = lane; i < nb; i += 32) s += prof[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        const float m = (float)(s / nb);
-        double s2 = 0;
-        for (int i = lane; i < nb; i += 32) {
-            const float p = prof[i] - m;
-            prof[i] = p;
-            s2 += (double)(p * p);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-        const double inv = 1.0 / sqrt(s2 / nb);
-        for (int i = lane; i < nb; i += 32) prof[i] = (float)((double)prof[i] * inv);
-    }
-    __syncthreads();
+    constexpr float c16[4] = {1.0f, 0.92387953251128675613f, 0.70710678118654752440f, 0.38268343236508977173f};
+    constexpr int j = J * (16 / N);  // sixteenths of a turn, 0 .. 7
+    if constexpr (j == 0) return z;
+    if constexpr (j == 4) return conj ? make_float2(-z.y, z.x) : make_float2(z.y, -z.x);
+    constexpr float wr = j < 4 ? c16[j & 3] : -c16[(8 - j) & 3];
+    constexpr float wi = -(j < 4 ? c16[(4 - j) & 3] : c16[(j - 4) & 3]);
+    const float s = conj ? -wi : wi;
+    return make_float2(z.x * wr - z.y * s, z.x * s + z.y * wr);
 }
 
-// One plane's score of CPUTracker::LUTProfileCompare (cpu_tracker.cpp:820-830) in the reference's
-// arithmetic and order: d = (double)(p_r - L_kr) with the difference taken in FP32, d *= w_r,
-// then sum += -(d * d) over r = 0 .. nb-1 in FP64, every operation rounded on its own (no
-// contraction). Given the same profile, the score equals the reference's bit for bit.
-// lut_k[r * stride] is L_kr.
-__device__ __forceinline__ double zlut_score(const float *prof, const float *lut_k, int stride, const float *w, int nb)
+template <int E, int H, int I = 0>
+__device__ __forceinline__ void lane_dif_stage(float2 (&z)[E])
 {
-    double acc = 0.0;
+    if constexpr (I < E) {
+        if constexpr ((I & H) == 0) {
+            const float2 a = z[I], b = z[I + H];
+            z[I] = make_float2(a.x + b.x, a.y + b.y);
+            z[I + H] = cmul_root<2 * H, I & (H - 1)>(make_float2(a.x - b.x, a.y - b.y), false);
+        }
+        lane_dif_stage<E, H, I + 1>(z);
+    }
+}
+
+template <int E, int H, int I = 0>
+__device__ __forceinline__ void lane_dit_stage(float2 (&z)[E])
+{
+    if constexpr (I < E) {
+        if constexpr ((I & H) == 0) {
+            const float2 a = z[I], b = cmul_root<2 * H, I & (H - 1)>(z[I + H], true);
+            z[I] = make_float2(a.x + b.x, a.y + b.y);
+            z[I + H] = make_float2(a.x - b.x, a.y - b.y);
+        }
+        lane_dit_stage<E, H, I + 1>(z);
+    }
+}
+
+template <int E, int H = E / 2>
+__device__ __forceinline__ void lane_dif(float2 (&z)[E])
+{
+    if constexpr (H >= 1) {
+        lane_dif_stage<E, H>(z);
+        lane_dif<E, H / 2>(z);
+    }
+}
+
+template <int E, int H = 1>
+__device__ __forceinline__ void lane_dit(float2 (&z)[E])
+{
+    if constexpr (H < E) {
+        lane_dit_stage<E, H>(z);
+        lane_dit<E, 2 * H>(z);
+    }
+}
+
+__device__ __forceinline__ float2 shfl2(float2 v, int src)
+{
+    return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
+__device__ __forceinline__ float2 shfl2_xor(float2 v, int o)
+{
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+
+// tw[k] = e^{-2 pi i k / L}, k < L/2. On return z[e] of lane l is (out_x[n], out_y[n]) at n = l + 32 e.
+template <int E>
+__device__ __forceinline__ void qi_autoconv_regs(const float2 *A, const float2 *tw, float2 (&z)[E])
+{
+    constexpr int L = 32 * E, lE = E == 1 ? 0 : (E == 2 ? 1 : (E == 4 ? 2 : (E == 8 ? 3 : 4)));
+    const int lane = threadIdx.x & 31;
+    auto root = [&](int k) {  // e^{-2 pi i k / L}, k < L
+        const float2 w = tw[k & (L / 2 - 1)];
+        return k & (L / 2) ? make_float2(-w.x, -w.y) : w;
+    };
+#pragma unroll
+    for (int e = 0; e < E; e++) z[e] = A[lane + 32 * e];
+    float2 t[4];  // twiddles of the lane distances 16, 8, 4, 2 (1 for the lanes that keep the sum)
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        const int d = 16 >> s;
+        t[s] = (lane & d) ? tw[((lane & (d - 1)) << s) * E] : make_float2(1.0f, 0.0f);
+    }
+    lane_dif<E>(z);
+#pragma unroll
+    for (int e = 1; e < E; e++) z[e] = cmul(z[e], root(lane * bitrev_c(e, lE)));
+#pragma unroll
+    for (int s = 0; s < 5; s++) {
+        const int d = 16 >> s;
+        const float sg = (lane & d) ? -1.0f : 1.0f;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const float2 o = shfl2_xor(z[e], d);
+            z[e] = make_float2(fmaf(sg, z[e].x, o.x), fmaf(sg, z[e].y, o.y));
+            if (s < 4) z[e] = cmul(z[e], t[s]);
+        }
+    }
+    // split the packed transform (see qi_autoconv_fft_filled): the conjugate frequency L - k lies in the
+    // mirrored lane's slot E - q, for q = 0 in its own slot of the lane that holds -m mod 32
+    const int m = (int)bitrev(lane, 5), opp = (int)bitrev((32 - m) & 31, 5);
+    float2 p[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const int q = bitrev_c(e, lE);
+        const float2 Zk = z[e], Zc = q == 0 ? shfl2(z[0], opp) : shfl2_xor(z[bitrev_c((E - q) & (E - 1), lE)], 31);
+        const float2 Px = make_float2(0.5f * (Zk.x + Zc.x), 0.5f * (Zk.y - Zc.y));
+        const float2 Py = make_float2(0.5f * (Zk.y + Zc.y), -0.5f * (Zk.x - Zc.x));
+        const float2 X = cmul(Px, Px), Y = cmul(Py, Py);
+        p[e] = cmul(root(q + E * m), make_float2(X.x - Y.y, X.y + Y.x));
+    }
+#pragma unroll
+    for (int s = 4; s >= 0; s--) {
+        const int d = 16 >> s;
+        const float sg = (lane & d) ? -1.0f : 1.0f;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const float2 v = s < 4 ? cmul(p[e], make_float2(t[s].x, -t[s].y)) : p[e];
+            const float2 o = shfl2_xor(v, d);
+            p[e] = make_float2(fmaf(sg, v.x, o.x), fmaf(sg, v.y, o.y));
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const float2 w = e > 0 ? root(lane * bitrev_c(e, lE)) : make_float2(1.0f, 0.0f);
+        z[e] = e > 0 ? cmul(p[e], make_float2(w.x, -w.y)) : p[e];
+    }
+    lane_dit<E>(z);
+}
+
+// warp_argmax over doubles: the keys' high and low words reduced in turn, then the smallest index.
+template <typename Get>
+__device__ __forceinline__ int warp_argmax_f64(Get at, int len)
+{
+    const int lane = threadIdx.x & 31;
+    long long best = (long long)0x8000000000000000ull;
+    int bi = 0x7fffffff;
+    for (int i = lane; i < len; i += 32) {
+        const double v = at(i) + 0.0;
+        long long k = __double_as_longlong(v);
+        k = v == v ? k ^ ((k >> 63) & 0x7fffffffffffffffll) : (long long)0x8000000000000000ull;
+        if (k > best) {
+            best = k;
+            bi = i;
+        }
+    }
+    const int hi = (int)(best >> 32), mhi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = hi == mhi ? (unsigned)best : 0u, mlo = __reduce_max_sync(0xffffffffu, lo);
+    bi = __reduce_min_sync(0xffffffffu, hi == mhi && lo == mlo ? bi : 0x7fffffff);
+    return bi == 0x7fffffff ? 0 : bi;
+}
+
+// A float as a signed integer of the same order; NaN below everything, -0 with +0.
+__device__ __forceinline__ int order_key(float v)
+{
+    const int b = __float_as_int(v + 0.0f);
+    return v == v ? b ^ ((b >> 31) & 0x7fffffff) : (int)0x80000000;
+}
+
+// The score of CPUTracker::LUTProfileCompare (cpu_tracker.cpp:820-830): -sum_r d^2 with d = (double)(p_r -
+// L_kr), the difference taken in FP32 as the reference takes it, then d *= w_r, summed in FP64. The bins are
+// cut into zlut_runs(planes) runs whose sums meet pairwise (0+1, 2+3, ...), in this order wherever a score
+// is formed, so that it does not depend on which kernel asks (FP64 rounding differs from a single run's
+// by about 1e-16 of the sum).
+// Runs: 1, 2, 4 or 8 neighbouring threads share four planes as long as 128 threads suffice for all planes.
+__device__ __forceinline__ int zlut_log2_runs(int planes)
+{
+    int lg = 0;
+    while (lg < 3 && ((planes + 3) >> 2) << (lg + 1) <= 128) lg++;
+    return lg;
+}
+
+// One plane's score; lut_k[r] is L_kr.
+__device__ __forceinline__ double zlut_score(const float *prof, const float *lut_k, const float *w, int nb, int planes)
+{
+    const int lg = zlut_log2_runs(planes), len = (nb + (1 << lg) - 1) >> lg;
+    double part[3] = {0.0, 0.0, 0.0}, v = 0.0;  // part: pending sums of 1, 2 and 4 runs
+    for (int s = 0; s < 1 << lg; s++) {
+        v = 0.0;
+        const int end = min(nb, (s + 1) * len);
 #pragma unroll 8
-    for (int r = 0; r < nb; r++) {
-        double d = (double)(prof[r] - __ldg(lut_k + (size_t)r * stride));
-        if (w) d = __dmul_rn(d, (double)__ldg(w + r));
-        acc = __dadd_rn(acc, -__dmul_rn(d, d));
+        for (int r = s * len; r < end; r++) {
+            double d = (double)(prof[r] - __ldg(lut_k + r));
+            if (w) d *= (double)__ldg(w + r);
+            v = fma(d, d, v);
+        }
+        if (s & 1) v = part[0] + v;
+        if ((s & 3) == 3) v = part[1] + v;
+        if ((s & 7) == 7) v = part[2] + v;
+        if (!(s & 1)) part[0] = v;
+        if ((s & 3) == 1) part[1] = v;
+        if ((s & 7) == 3) part[2] = v;
     }
-    return acc;
+    return -v;
 }
 
-// The plain Z match: one thread per plane, reading the transposed LUT ([bin][plane], `pitch`
-// planes per bin) so that a warp's 32 planes are one coalesced 128-byte load per bin.
-__device__ inline void zlut_scores_plain(const float *prof, const float *lut_t, int pitch, int planes, int nb,
-                                         const float *weights, double *scores)
+// The plain Z match over the transposed LUT ([bin][plane], `pitch` planes per bin, a multiple of 32): a thread
+// takes four planes (16-byte loads, four independent FP64 chains) over one run of bins. What a thread waits for
+// is the LUT (L2): one thread per plane over all bins in turn took 17.2 k of a 100x100 ROI's 146 k cycles (200 planes
+// x 64 bins, 128 threads, full load), this 7.1 k.
+template <bool kWeights>
+__device__ __forceinline__ void zlut_scores_runs(const float *prof, const float4 *lut4, int pitch4, int planes, int nb,
+                                                 const float *weights, double *scores)
 {
-    for (int k = threadIdx.x; k < planes; k += blockDim.x) scores[k] = zlut_score(prof, lut_t + k, pitch, weights, nb);
+    const int quads = (planes + 3) >> 2, lg = zlut_log2_runs(planes), len = (nb + (1 << lg) - 1) >> lg;
+    const int total = quads << lg;
+    for (int base = 0; base < total; base += blockDim.x) {  // uniform: the sums below shuffle whole warps
+        const int t = base + threadIdx.x;
+        if ((t & ~31) >= total) break;  // whole warps
+        const int q = min(t >> lg, quads - 1), h = t & ((1 << lg) - 1);
+        const int r0 = h * len, r1 = min(nb, r0 + len);
+        const float4 *l = lut4 + (size_t)r0 * pitch4 + q;
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+        for (int r = r0; r < r1; r++, l += pitch4) {
+            const float4 f = __ldg(l);
+            const float p = prof[r];
+            double d[4] = {(double)(p - f.x), (double)(p - f.y), (double)(p - f.z), (double)(p - f.w)};
+            const double w = kWeights ? (double)__ldg(weights + r) : 1.0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                if (kWeights) d[i] *= w;
+                v[i] = fma(d[i], d[i], v[i]);
+            }
+        }
+        for (int o = 1; o < 1 << lg; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        if (t < total && h == 0)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (4 * q + i < planes) scores[4 * q + i] = -v[i];
+    }
     __syncthreads();
+}
+
+__device__ __forceinline__ void zlut_scores_plain(const float *prof, const float *lut_t, int pitch, int planes, int nb,
+                                                  const float *weights, double *scores)
+{
+    const float4 *lut4 = reinterpret_cast<const float4 *>(lut_t);
+    if (weights)
+        zlut_scores_runs<true>(prof, lut4, pitch >> 2, planes, nb, weights, scores);
+    else
+        zlut_scores_runs<false>(prof, lut4, pitch >> 2, planes, nb, weights, scores);
 }
 
 // QueuedTracker::ZLUTBiasCorrection, cputrack/QueuedTracker.cpp:115-140: four fixed-point steps

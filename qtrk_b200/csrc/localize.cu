@@ -1,9 +1,9 @@
 // Localization kernels for sm_100a.
 //
 // localize_qi_kernel: one CTA per ROI runs the whole per-ROI pipeline of
-//   QueuedCPUTracker::ProcessJob (cputrack/QueuedCPUTracker.cpp:273-361) on a float tile of the
-//   ROI in shared memory: bulk copy (or batched loads) + convert (+ calibration) fused with the
-//   first COM pass -> COM -> QI iterations -> radial profile -> Z-LUT match -> result. Pixels are
+//   QueuedCPUTracker::ProcessJob (cputrack/QueuedCPUTracker.cpp:273-361) on a tile of the ROI in
+//   shared memory (tile.cuh): bulk copy (or batched loads) + convert (+ calibration) fused with the
+//   pixel sum -> COM -> QI iterations -> radial profile -> Z-LUT match -> result. Pixels are
 //   read from HBM exactly once; everything after the load works on-chip.
 // localize_gauss_kernel: one CTA per ROI, COM -> 2D Gaussian MLE (-> Z) on a plain tile.
 // build_lut_kernel / finalize_lut_kernel: QueuedCPUTracker::BuildLUT / FinalizeLUT
@@ -16,9 +16,8 @@
 
 #include <cuda_bf16.h>
 
-#include "bulk_copy.cuh"
-#include "device_common.cuh"
 #include "kernels.h"
+#include "tile.cuh"
 
 namespace qtrk {
 
@@ -27,7 +26,8 @@ __device__ const float kQIWeights[7] = {0.14f, 0.5f, 0.85f, 1.0f, 0.85f, 0.5f, 0
 __device__ const float kZLUTWeights[7] = {0.15f, 0.5f, 0.85f, 1.0f, 0.85f, 0.5f, 0.15f};
 
 struct SmemView {
-    float *img, *misc;
+    uint32_t *img;  // the tile (tile.cuh)
+    float *misc;
     float4 *qdirs;  // QI quadrant directions as (d.x, d.x, d.y, d.y)
     float2 *tw;
     float4 *zdirs;  // full-circle directions in pairs (j, j + n/2), see load_z_tables
@@ -39,7 +39,7 @@ struct SmemView {
 __device__ __forceinline__ SmemView smem_view(uint8_t *smem, const TrackParams &P)
 {
     SmemView v;
-    v.img = reinterpret_cast<float *>(smem + P.sm_img);
+    v.img = reinterpret_cast<uint32_t *>(smem + P.sm_img);
     v.misc = reinterpret_cast<float *>(smem + P.sm_misc);
     v.red = reinterpret_cast<double *>(smem + P.sm_red);
     v.work = smem + P.sm_work;
@@ -47,7 +47,7 @@ __device__ __forceinline__ SmemView smem_view(uint8_t *smem, const TrackParams &
     v.qdirs = reinterpret_cast<float4 *>(tab);
     v.tw = tab + 2 * P.qi_angpq;  // L/2 = qi_nr twiddles
     v.qrw = reinterpret_cast<float *>(v.tw + P.qi_nr);
-    v.zdirs = reinterpret_cast<float4 *>(tab);  // loaded over the QI tables once QI is done
+    v.zdirs = reinterpret_cast<float4 *>(smem + P.sm_zdirs);
     return v;
 }
 
@@ -68,8 +68,8 @@ __device__ __forceinline__ void load_qi_tables(const SmemView &s, const TrackPar
         for (int i = threadIdx.x; i < P.qi_nr; i += blockDim.x) s.qrw[i] = P.qi_rweights[i];
 }
 
-// Copy the full-circle direction table over the QI tables (all threads; the QI stage must
-// be finished, and a barrier must follow before use).
+// Copy the full-circle direction table (all threads; a barrier must follow before use). Where shared memory
+// is short (sm_zdirs == sm_tables) it goes over the QI tables, and the QI stage must be finished.
 __device__ __forceinline__ void load_z_tables(const SmemView &s, const TrackParams &P)
 {
     const float2 *zd = static_cast<const float2 *>(P.z_dirs);
@@ -85,43 +85,15 @@ __device__ __forceinline__ void load_z_tables(const SmemView &s, const TrackPara
 }
 
 // The QI position update from the two autoconvolutions (cpu_tracker.cpp:345-357, 400-410):
-// ComputeMaxInterp over autoconv[x] = ac[(x + nr) mod L] for X (.x) and Y (.y), by one warp: a
-// two-axis argmax over the warp (first index of the maximum, as warp_argmax), then the 7-point
-// fits of both axes side by side (even lanes X, odd lanes Y). Lanes 0 and 1 write the new x and y
-// to misc[0] and misc[1]. Runs on the warp that made ac, right after it, with no CTA barrier.
-__device__ __forceinline__ void qi_fit_xy(const float2 *ac, int nr, float cx, float cy, float rstep, float *misc)
+// ComputeMaxInterp over autoconv[x] = ac[(x + nr) mod L] for X (.x) and Y (.y), by one warp, given the
+// first indices ix, iy of the maxima: the 7-point fits of both axes side by side (even lanes X, odd
+// lanes Y). Lanes 0 and 1 write the new x and y to misc[0] and misc[1].
+__device__ __noinline__ void qi_fit_at(const float2 *ac, int nr, int ix, int iy, float cx, float cy, float rstep,
+                                       float *misc)
 {
+    __builtin_assume(__isShared(ac));
+    __builtin_assume(__isShared(misc));
     const int lane = threadIdx.x & 31, L = 2 * nr;
-    float bx = 0.0f, by = 0.0f;
-    int ix = -1, iy = -1;
-    for (int x = lane; x < L; x += 32) {
-        int n = x + nr;
-        if (n >= L) n -= L;
-        const float2 v = ac[n];
-        if (v.x == v.x && (ix < 0 || v.x > bx)) {
-            bx = v.x;
-            ix = x;
-        }
-        if (v.y == v.y && (iy < 0 || v.y > by)) {
-            by = v.y;
-            iy = x;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ox = __shfl_xor_sync(0xffffffffu, bx, o), oy = __shfl_xor_sync(0xffffffffu, by, o);
-        const int oix = __shfl_xor_sync(0xffffffffu, ix, o), oiy = __shfl_xor_sync(0xffffffffu, iy, o);
-        if (oix >= 0 && (ix < 0 || ox > bx || (ox == bx && oix < ix))) {
-            bx = ox;
-            ix = oix;
-        }
-        if (oiy >= 0 && (iy < 0 || oy > by || (oy == by && oiy < iy))) {
-            by = oy;
-            iy = oiy;
-        }
-    }
-    ix = ix < 0 ? 0 : ix;
-    iy = iy < 0 ? 0 : iy;
     const bool yaxis = (lane & 1) != 0;
     float m;
     if (ix >= 3 && ix + 4 <= L && iy >= 3 && iy + 4 <= L) {  // both windows inside: per-lane fits
@@ -152,31 +124,84 @@ __device__ __forceinline__ void qi_fit_xy(const float2 *ac, int nr, float cx, fl
     }
 }
 
+// Transform, argmax and fit with the autoconvolutions in registers (L = 32 E): the maximum of each axis by
+// one integer warp reduction over order_key, its first index by another (as the strict ">" scan of
+// LsqQuadraticFit.h:140-147 finds it; NaN never wins). The result replaces the profile in A, for the fit's
+// windows (every lane has read its elements before the first shuffle).
+template <int E>
+__device__ __noinline__ void qi_update_regs(float2 *A, const float2 *tw, float cx, float cy, float rstep, float *misc)
+{
+    __builtin_assume(__isShared(A));  // not inlined: its pointers' address space is not seen otherwise
+    __builtin_assume(__isShared(tw));
+    constexpr int L = 32 * E, nr = L / 2;
+    const int lane = threadIdx.x & 31;
+    float2 z[E];
+    qi_autoconv_regs<E>(A, tw, z);
+    int kx = (int)0x80000000, ky = kx;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        A[lane + 32 * e] = z[e];
+        kx = max(kx, order_key(z[e].x));
+        ky = max(ky, order_key(z[e].y));
+    }
+    kx = __reduce_max_sync(0xffffffffu, kx);
+    ky = __reduce_max_sync(0xffffffffu, ky);
+    int ix = L, iy = L;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const int x = (lane + 32 * e + nr) & (L - 1);
+        if (order_key(z[e].x) == kx) ix = min(ix, x);
+        if (order_key(z[e].y) == ky) iy = min(iy, x);
+    }
+    ix = __reduce_min_sync(0xffffffffu, ix);
+    iy = __reduce_min_sync(0xffffffffu, iy);
+    __syncwarp();
+    qi_fit_at(A, nr, ix, iy, cx, cy, rstep, misc);
+}
+
+// The same for the other lengths (2 nr < 32 or > 512), through shared memory; A in bit-reversed order.
+__device__ __noinline__ void qi_update_smem(float2 *A, float2 *ac, int nr, const float2 *tw, float cx, float cy,
+                                            float rstep, float *misc)
+{
+    const int L = 2 * nr;
+    qi_autoconv_fft_filled(nr, A, ac, tw);
+    auto at = [&](int x, bool yaxis) {
+        int n = x + nr;
+        if (n >= L) n -= L;
+        return yaxis ? ac[n].y : ac[n].x;
+    };
+    const int ix = warp_argmax([&](int x) { return at(x, false); }, L);
+    const int iy = warp_argmax([&](int x) { return at(x, true); }, L);
+    qi_fit_at(ac, nr, ix, iy, cx, cy, rstep, misc);
+}
+
 // CPUTracker::ComputeQI, cpu_tracker.cpp:285-360. All threads call; returns the position and the
 // boundary flag of the last iteration.
-__device__ void qi_localize(const SmemView &s, const TrackParams &P, float mean, float &cx, float &cy, bool &bhit,
-                            const float *rweights)
+template <int F, int T>
+__device__ __forceinline__ void qi_localize(const SmemView &s, const TrackParams &P, float mean, float &cx, float &cy,
+                                            bool &bhit, const float *rweights)
 {
     const int W = P.width, H = P.height, nr = P.qi_nr, L = 2 * nr;
-    const bool pow2 = (L & (L - 1)) == 0 && L >= 2;
-    // work: [ ac (L complex) ] [ A (L complex) ] [ subset partials (2 KB) ]
-    float2 *ac = reinterpret_cast<float2 *>(s.work);
-    float2 *A = reinterpret_cast<float2 *>(s.work + L * 8);
-    float4 *part = reinterpret_cast<float4 *>(s.work + 2 * L * 8);
+    const bool regs = L >= 32 && L <= 512;  // L is a power of two
+    // work: [ A (L complex) ] [ ac (L complex), only for the transform through shared memory ]
+    float2 *A = reinterpret_cast<float2 *>(s.work);
     const float rstep = (P.qi_maxr - P.qi_minr) / (float)nr;  // also pixelsPerProfLen (cpu_tracker.cpp:311,649)
+#pragma unroll 1
     for (int k = 0; k < P.qi_iterations; k++) {
         bhit = check_boundaries(cx, cy, P.qi_maxr, W, H);
-        qi_profiles_sym(s.img, W, H, W, cx, cy, mean, nr, P.qi_nang[k], P.qi_inv_nang[k], P.qi_stride[k], P.qi_minr, rstep,
-                        s.qdirs, rweights, part, A, pow2 ? ilog2_pow2(L) : -1);
+        qi_profiles<F, T>(s.img, W, H, P.tile_pitch, cx, cy, mean, nr, P.qi_nang[k], P.qi_inv_nang[k], P.qi_stride[k],
+                          P.qi_minr, rstep, s.qdirs, rweights, A, regs ? -1 : ilog2_pow2(L));
         __syncthreads();
-        if (pow2) {
-            if (threadIdx.x < 32) {  // transform and fits on warp 0, the others wait at the next barrier
-                qi_autoconv_fft_filled(nr, A, ac, s.tw);
-                qi_fit_xy(ac, nr, cx, cy, rstep, s.misc);
+        if (threadIdx.x < 32) {  // transform and fits on warp 0, the others wait at the next barrier
+            __syncwarp();        // its shuffles run as one warp (a lane that diverged earlier may still be apart)
+            switch (L) {
+            case 32: qi_update_regs<1>(A, s.tw, cx, cy, rstep, s.misc); break;
+            case 64: qi_update_regs<2>(A, s.tw, cx, cy, rstep, s.misc); break;
+            case 128: qi_update_regs<4>(A, s.tw, cx, cy, rstep, s.misc); break;
+            case 256: qi_update_regs<8>(A, s.tw, cx, cy, rstep, s.misc); break;
+            case 512: qi_update_regs<16>(A, s.tw, cx, cy, rstep, s.misc); break;
+            default: qi_update_smem(A, A + L, nr, s.tw, cx, cy, rstep, s.misc);
             }
-        } else {
-            qi_autoconv_direct_filled(nr, A, ac);
-            if (threadIdx.x < 32) qi_fit_xy(ac, nr, cx, cy, rstep, s.misc);
         }
         __syncthreads();
         // misc[0..1] is written again only after the next iteration's first barrier, which every
@@ -188,16 +213,20 @@ __device__ void qi_localize(const SmemView &s, const TrackParams &P, float mean,
 
 // Radial profile + Z-LUT compare (QueuedCPUTracker.cpp:319-338). Returns z (0 without a LUT). With
 // P.zprof_f32 set, the profile is written out for the tensor-core match instead.
-__device__ float z_localize(const SmemView &s, const TrackParams &P, float mean, float x, float y, int bead, int roi)
+template <int F, int T>
+__device__ __forceinline__ float z_localize(const SmemView &s, const TrackParams &P, int ts, float mean, float x, float y,
+                                            int bead, int roi)
 {
     const int nb = P.z_nbins;
     float *prof = reinterpret_cast<float *>(s.work);
     double *scores = reinterpret_cast<double *>(s.work + (((nb * 4) + 15) & ~15));
     const float rstep = (P.z_maxr - P.z_minr) / (float)nb;
-    load_z_tables(s, P);
-    __syncthreads();
-    radial_profile(s.img, P.width, P.height, P.width, x, y, mean, nb, P.z_angsteps, P.z_minr, rstep, s.zdirs, prof,
-                   (P.mode & kLT_NormalizeProfile) != 0, s.red);
+    if (P.sm_zdirs == P.sm_tables) {
+        load_z_tables(s, P);
+        __syncthreads();
+    }
+    radial_profile<F, T>(s.img, P.width, P.height, ts, x, y, mean, nb, P.z_angsteps, P.z_minr, rstep, s.zdirs, prof,
+                         (P.mode & kLT_NormalizeProfile) != 0);
     if (P.zprof_f32) {
         // [hi | lo] BF16 split of the weighted profile: v = hi + lo + O(2^-16 v)
         __nv_bfloat16 *pb = static_cast<__nv_bfloat16 *>(P.zprof_bf16) + (size_t)roi * 2 * P.zprof_nbp;
@@ -222,8 +251,9 @@ __device__ float z_localize(const SmemView &s, const TrackParams &P, float mean,
         for (int k = threadIdx.x; k < P.lut_planes; k += blockDim.x)
             P.cmp_scores[(size_t)bead * P.lut_planes + k] = (float)scores[k];
     if (threadIdx.x < 32) {
+        __syncwarp();
         auto at = [&](int i) { return scores[i]; };
-        const int im = warp_argmax(at, P.lut_planes);
+        const int im = warp_argmax_f64(at, P.lut_planes);
         const float z = max_interp7_sym(at, P.lut_planes, im, kZLUTWeights);
         if (threadIdx.x == 0) s.misc[2] = zlut_bias_correct(z, P.lut_planes, P.zbias, P.zbias_w, P.zbias_count, bead);
     }
@@ -231,19 +261,60 @@ __device__ float z_localize(const SmemView &s, const TrackParams &P, float mean,
     return s.misc[2];
 }
 
-constexpr int kMinBlocks = 5;  // CTAs per SM the QI and Gaussian kernels are compiled for (<= 96 registers)
+// CTAs per SM the 128-thread kernels are compiled for (72 registers): ROIs of up to about 80 px fit seven times,
+// and a frame of 1,000 then runs in one wave (60x60 f32: 57 us, 70 us with five CTAs of 96 registers; 64x64 u16: 55
+// and 64 us); larger ROIs, five to an SM by their tiles, lose 1 % (10,000 of 100x100: 842 and 834 us).
+constexpr int kMinBlocks = 7;
 
 constexpr uint32_t kStageWaitLimit = 1u << 22;  // mbarrier polls before a staged copy counts as lost
 
-// COM / QI (+ Z): QueuedCPUTracker::ProcessJob (QueuedCPUTracker.cpp:273-361), one CTA per ROI.
-// The ROI becomes a float tile in shared memory. With kStaged (ROIs back to back, 16-byte
-// aligned, whole 16-byte chunks) its raw bytes arrive by one bulk copy (cp.async.bulk, completion
-// on an mbarrier) started by thread 0 as the CTA begins, while the other threads fetch the QI
-// tables, and are converted in place; otherwise the threads load them with batched streaming
-// loads (frame bands, unaligned ROIs). The COM's first pass is fused into either conversion.
-// One instantiation per form, so neither carries the other's registers.
-template <bool kStaged>
-__global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
+// Bring ROI bytes at `src` into the tile and measure mean and COM. A contiguous ROI arrives by one bulk copy
+// (cp.async.bulk, completion on an mbarrier) that thread 0 starts first, while the others fetch the tables;
+// its up to 15 bytes before and behind the whole 16-byte units are loaded directly. Frame bands, and
+// small or misaligned ROIs, are loaded row by row.
+template <int F, int T>
+__device__ __forceinline__ ComResult load_tile(const SmemView &s, const TrackParams &P, const uint8_t *src, int pitch,
+                                               int bead, float bgcorr)
+{
+    const int W = P.width, H = P.height, bpp = tile_bpp(P), bytes = W * H * bpp, ts = P.tile_pitch;
+    const int misalign = (int)(reinterpret_cast<uintptr_t>(src) & 15);
+    if (F == kTileF32 && packed_rows(W, ts)) {  // the largest odd ROIs: a tile without room for padded rows
+        load_qi_tables(s, P);
+        const BlockGroup g{s.red};
+        float *img = reinterpret_cast<float *>(s.img);
+        return com_from_sums(g, img, W, H, load_roi(g, img, src, pitch, P, bead), bgcorr);
+    }
+    const bool bulk = pitch == W * bpp && bytes >= kMinBulkBytes && !(misalign & (bpp - 1));
+    uint8_t *raw = reinterpret_cast<uint8_t *>(s.img) + raw_offset(W, H, ts, bpp, bulk ? misalign : 0);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(s.misc) + 32);
+    if (bulk && threadIdx.x == 0) {
+        mbar_init(mbar);
+        bulk_load_inner(raw, src, bytes, mbar);
+    }
+    load_qi_tables(s, P);
+    if (P.sm_zdirs != P.sm_tables) load_z_tables(s, P);
+    if (bulk) {
+        load_ends(raw, src, bytes);
+        // one thread waits for the copy (its acquire, then the barrier, order the copied bytes
+        // before every thread's reads); the others wait at the barrier without polling
+        if (threadIdx.x == 0 && !mbar_wait(mbar, 0, kStageWaitLimit) && P.err_flag) atomicOr(P.err_flag, 4u);
+    } else {
+        load_rows<T>(raw, src, pitch, W * bpp, H);
+    }
+    __syncthreads();
+    if (F != kTileF32 && (P.mode & kLT_ClearFirstFourPixels)) {  // QueuedCPUTracker.cpp:280-282
+        if (threadIdx.x < 4 * bpp) raw[threadIdx.x] = 0;
+        __syncthreads();
+    }
+    uint32_t isum;
+    const double sum = convert_raw<F, T>(s.img, raw, ts, P, bead, isum);
+    return tile_com<F, T>(s.img, W, H, ts, sum, isum, bgcorr, s.red);
+}
+
+// COM / QI (+ Z): QueuedCPUTracker::ProcessJob (QueuedCPUTracker.cpp:273-361), one CTA of T threads per
+// ROI on a tile of format F.
+template <int F, int T>
+__global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
     localize_qi_kernel(TrackParams P, const uint8_t *__restrict__ pixels, int pitch, int64_t roi_stride,
                        const int64_t *__restrict__ roi_offsets, const LocalizationJob *__restrict__ jobs, int count,
                        LocalizationResult *__restrict__ results)
@@ -253,32 +324,10 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     if (roi >= count) return;
     const SmemView s = smem_view(smem, P);
     const int W = P.width, H = P.height;
-    BlockGroup g{s.red};
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(s.misc) + 32);
-    if constexpr (kStaged) {
-        if (threadIdx.x == 0) {
-            const int bpp = P.pdt == 0 ? 1 : (P.pdt == 1 ? 2 : 4);
-            const int n = W * H;
-            mbar_init(mbar);
-            bulk_load(reinterpret_cast<uint8_t *>(s.img) + (size_t)(4 - bpp) * n, pixels + (int64_t)roi * roi_stride,
-                      (uint32_t)(bpp * n), mbar);
-        }
-    }
     // the job's words are read again for the result (no registers held through QI and Z)
     const int bead = jobs ? (int)reinterpret_cast<const uint32_t *>(jobs)[(size_t)roi * 6 + 2] : 0;
-    load_qi_tables(s, P);
-    float2 part;
-    if constexpr (kStaged) {
-        // one thread waits for the copy (its acquire, then the barrier, order the copied bytes
-        // before every thread's reads); the others wait at the barrier without polling
-        if (threadIdx.x == 0 && !mbar_wait(mbar, 0, kStageWaitLimit) && P.err_flag) atomicOr(P.err_flag, 4u);
-        __syncthreads();
-        part = convert_staged(g, s.img, P, bead);
-    } else {
-        const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
-        part = load_roi(g, s.img, pixels + off, pitch, P, bead);
-    }
-    const ComResult com = com_from_sums(g, s.img, W, H, part, P.com_bgcorrection);
+    const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
+    const ComResult com = load_tile<F, T>(s, P, pixels + off, pitch, bead, P.com_bgcorrection);
     float comx = com.x, comy = com.y;
     if (isnan(comx) || isnan(comy)) {  // QueuedCPUTracker.cpp:294-295
         comx = (float)(W / 2);
@@ -286,10 +335,10 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     }
     float x = comx, y = comy, z = 0.0f;
     bool bhit = false;
-    if (P.mode & kLT_QI) qi_localize(s, P, com.mean, x, y, bhit, P.qi_rweights ? s.qrw : nullptr);
+    if (P.mode & kLT_QI) qi_localize<F, T>(s, P, com.mean, x, y, bhit, P.qi_rweights ? s.qrw : nullptr);
     if (P.mode & kLT_LocalizeZ) {
         bhit = check_boundaries(x, y, P.z_maxr, W, H);
-        z = z_localize(s, P, com.mean, x, y, bead, roi);
+        z = z_localize<F, T>(s, P, P.tile_pitch, com.mean, x, y, bead, roi);
     }
     if (threadIdx.x == 0) {
         uint32_t job[6];
@@ -315,8 +364,9 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
     BlockGroup g{s.red};
     const int W = P.width, H = P.height;
-    const float2 part = load_roi(g, s.img, pixels + off, pitch, P, bead);
-    const ComResult com = com_from_sums(g, s.img, W, H, part, P.com_bgcorrection);
+    float *img = reinterpret_cast<float *>(s.img);
+    const float2 part = load_roi(g, img, pixels + off, pitch, P, bead);
+    const ComResult com = com_from_sums(g, img, W, H, part, P.com_bgcorrection);
     float comx = com.x, comy = com.y;
     if (isnan(comx) || isnan(comy)) {  // QueuedCPUTracker.cpp:294-295
         comx = (float)(W / 2);
@@ -327,17 +377,21 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     float *col = reinterpret_cast<float *>(s.work);
     if (P.mode & kLT_Gaussian5P) {
         float p[5] = {x, y, com.mean * 0.5f * (float)(W * H), com.mean * 0.5f, P.g_sigma};
-        gauss5_mle(g, s.img, W, H, p, P.g_iterations, col, col + 3 * W);
+        gauss5_mle(g, img, W, H, p, P.g_iterations, col, col + 3 * W);
         x = p[0];
         y = p[1];
         z = p[4];
     } else {
-        gauss4_mle(g, s.img, W, H, com.mean, x, y, P.g_iterations, P.g_sigma, col, col + 3 * W);
+        gauss4_mle(g, img, W, H, com.mean, x, y, P.g_iterations, P.g_sigma, col, col + 3 * W);
     }
     __syncthreads();
     if (P.mode & kLT_LocalizeZ) {
+        if (P.sm_zdirs != P.sm_tables) {
+            load_z_tables(s, P);
+            __syncthreads();
+        }
         bhit = check_boundaries(x, y, P.z_maxr, W, H);
-        z = z_localize(s, P, com.mean, x, y, bead, roi);
+        z = z_localize<kTileF32, kBlockThreads>(s, P, W, com.mean, x, y, bead, roi);
     }
     if (threadIdx.x == 0) write_result(results, roi, job, x, y, z, comx, comy, bhit ? 1u : 0u, com.mean);
 }
@@ -346,40 +400,39 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
 // at data + pitch*H*i. Position from known_pos, else COM (no background correction) + QI
 // without radial weights (line 603). The profile's fallback value is the tracker's mean,
 // which SetImage resets to 0 when known_pos skips the COM (cpu_tracker.h:135).
-__global__ void __launch_bounds__(kBlockThreads) build_lut_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
-                                                                  int pitch, int nbeads, int plane,
-                                                                  const float2 *__restrict__ known_pos,
-                                                                  int normalize, float *__restrict__ lut)
+template <int F, int T>
+__global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
+    build_lut_kernel(TrackParams P, const uint8_t *__restrict__ pixels, int pitch, int nbeads, int plane,
+                     const float2 *__restrict__ known_pos, int normalize, float *__restrict__ lut)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     const int bead = blockIdx.x;
     if (bead >= nbeads) return;
     const SmemView s = smem_view(smem, P);
-    load_qi_tables(s, P);
-    BlockGroup g{s.red};
-    const float2 part = load_roi(g, s.img, pixels + (size_t)pitch * P.height * bead, pitch, P, bead);
+    const ComResult com = load_tile<F, T>(s, P, pixels + (size_t)pitch * P.height * bead, pitch, bead, 0.0f);
     float x, y, mean = 0.0f;
     if (known_pos) {
         x = known_pos[bead].x;
         y = known_pos[bead].y;
     } else {
-        const ComResult com = com_from_sums(g, s.img, P.width, P.height, part, 0.0f);
         mean = com.mean;
         x = com.x;
         y = com.y;
         bool bhit;
-        qi_localize(s, P, mean, x, y, bhit, nullptr);
+        qi_localize<F, T>(s, P, mean, x, y, bhit, nullptr);
     }
     const int nb = P.z_nbins;
     float *prof = reinterpret_cast<float *>(s.work);
     const float rstep = (P.z_maxr - P.z_minr) / (float)nb;
     __syncthreads();
-    load_z_tables(s, P);
-    __syncthreads();
-    radial_profile(s.img, P.width, P.height, P.width, x, y, mean, nb, P.z_angsteps, P.z_minr, rstep, s.zdirs, prof,
-                   normalize != 0, s.red);
+    if (P.sm_zdirs == P.sm_tables) {
+        load_z_tables(s, P);
+        __syncthreads();
+    }
+    radial_profile<F, T>(s.img, P.width, P.height, P.tile_pitch, x, y, mean, nb, P.z_angsteps, P.z_minr, rstep, s.zdirs,
+                         prof, normalize != 0);
     float *dst = lut + ((size_t)bead * P.lut_planes + plane) * nb;
-    for (int r = threadIdx.x; r < nb; r += blockDim.x) dst[r] += prof[r];
+    for (int r = threadIdx.x; r < nb; r += T) dst[r] += prof[r];
 }
 
 // QueuedCPUTracker::FinalizeLUT (QueuedCPUTracker.cpp:648-659): NormalizeRadialProfile
@@ -416,11 +469,11 @@ __global__ void __launch_bounds__(kBlockThreads) profile_kernel(TrackParams P, c
     const SmemView s = smem_view(smem, P);
     load_z_tables(s, P);
     BlockGroup g{s.red};
-    load_roi(g, s.img, reinterpret_cast<const uint8_t *>(img_in), P.width * 4, P, -1);
+    load_roi(g, reinterpret_cast<float *>(s.img), reinterpret_cast<const uint8_t *>(img_in), P.width * 4, P, -1);
     float *prof = reinterpret_cast<float *>(s.work);
     const float rstep = (P.z_maxr - P.z_minr) / (float)P.z_nbins;
-    radial_profile(s.img, P.width, P.height, P.width, cx, cy, mean, P.z_nbins, P.z_angsteps, P.z_minr, rstep, s.zdirs,
-                   prof, normalize != 0, s.red);
+    radial_profile<kTileF32, kBlockThreads>(s.img, P.width, P.height, P.width, cx, cy, mean, P.z_nbins, P.z_angsteps,
+                                            P.z_minr, rstep, s.zdirs, prof, normalize != 0);
     for (int r = threadIdx.x; r < P.z_nbins; r += blockDim.x) out[r] = prof[r];
 }
 
@@ -429,25 +482,68 @@ __global__ void __launch_bounds__(kBlockThreads) profile_kernel(TrackParams P, c
 // ------------------------------------------------------------------------------------------
 static int align16(int v) { return (v + 15) & ~15; }
 
-void plan_smem(TrackParams &P)
+constexpr int kMaxSmem = 227 * 1024;
+
+// The layout of a localization CTA's shared memory. Where the padded rows and the separate direction tables do
+// not fit, rows are packed and the full-circle table goes over the QI tables.
+static void plan_smem_form(TrackParams &P, bool compact)
 {
     const int W = P.width, H = P.height;
     const int nr = P.qi_nr > 0 ? P.qi_nr : 1, L = 2 * nr;
     P.sm_img = 0;
-    P.sm_tables = align16(W * H * 4);
-    const int qi_tables = P.qi_angpq * 16 + nr * 8 + nr * 4, z_tables = ((P.z_angsteps + 1) >> 1) * 16;
-    P.sm_work = P.sm_tables + align16(qi_tables > z_tables ? qi_tables : z_tables);
-    // [ ac | A ] (L complex each) + 2 KB of subset partials when the QI directions are split over warps
-    const int qi_work = 2 * L * 8 + (nr < kBlockThreads / 4 ? 2048 : 0);
+    P.tile_pitch = compact ? W : tile_pitch(W);
+    P.sm_tables = tile_region_bytes(W, H, P.tile_pitch);
+    const int qi_tables = align16(P.qi_angpq * 16 + nr * 8 + nr * 4), z_tables = ((P.z_angsteps + 1) >> 1) * 16;
+    P.sm_zdirs = compact ? P.sm_tables : P.sm_tables + qi_tables;
+    P.sm_work = compact ? P.sm_tables + std::max(qi_tables, z_tables) : P.sm_zdirs + z_tables;
+    // QI: the profile (L complex), and its transform where that runs through shared memory
+    const int qi_work = (L >= 32 && L <= 512 ? 1 : 2) * L * 8;
     const int z_work = align16(P.z_nbins * 4) + P.lut_planes * 8;
-    const int g_work = (P.mode & kLT_Gaussian2D) ? (3 * W + 3 * H) * 4 : 0;
-    int work = qi_work;
-    if (z_work > work) work = z_work;
-    if (g_work > work) work = g_work;
-    P.sm_red = P.sm_work + align16(work);
-    constexpr int kRed = kBlockThreads / 32 * 20;  // block_sum scratch: N * warps doubles, N <= 20
-    P.sm_misc = P.sm_red + kRed * 8;
+    const bool gauss = (P.mode & kLT_Gaussian2D) != 0;
+    const int g_work = gauss ? (3 * W + 3 * H) * 4 : 0;
+    P.sm_red = P.sm_work + align16(std::max(qi_work, std::max(z_work, g_work)));
+    // block sum scratch, N * warps doubles: N <= 20 with 4 warps (Gaussian), 3 with up to 16
+    P.sm_misc = P.sm_red + (gauss ? 80 : 48) * 8;
     P.smem_bytes = P.sm_misc + 64;
+}
+
+void plan_smem(TrackParams &P)
+{
+    plan_smem_form(P, false);
+    if (P.smem_bytes > kMaxSmem) plan_smem_form(P, true);
+}
+
+// The kernel instantiations by tile format and threads per ROI.
+using QiKernel = void (*)(TrackParams, const uint8_t *, int, int64_t, const int64_t *, const LocalizationJob *, int,
+                          LocalizationResult *);
+using LutKernel = void (*)(TrackParams, const uint8_t *, int, int, int, const float2 *, int, float *);
+static const QiKernel kQiKernels[3][3] = {
+    {localize_qi_kernel<kTileF32, 128>, localize_qi_kernel<kTileF32, 256>, localize_qi_kernel<kTileF32, 512>},
+    {localize_qi_kernel<kTileU16, 128>, localize_qi_kernel<kTileU16, 256>, localize_qi_kernel<kTileU16, 512>},
+    {localize_qi_kernel<kTileU8, 128>, localize_qi_kernel<kTileU8, 256>, localize_qi_kernel<kTileU8, 512>}};
+static const LutKernel kLutKernels[3][3] = {
+    {build_lut_kernel<kTileF32, 128>, build_lut_kernel<kTileF32, 256>, build_lut_kernel<kTileF32, 512>},
+    {build_lut_kernel<kTileU16, 128>, build_lut_kernel<kTileU16, 256>, build_lut_kernel<kTileU16, 512>},
+    {build_lut_kernel<kTileU8, 128>, build_lut_kernel<kTileU8, 256>, build_lut_kernel<kTileU8, 512>}};
+
+// Integer pixels are packed unless calibration images turn them into fractions, or rows are.
+static int tile_format(const TrackParams &P)
+{
+    if (P.pdt == 2 || P.calib_count > 0 || packed_rows(P.width, P.tile_pitch)) return kTileF32;
+    return P.pdt == 1 ? kTileU16 : kTileU8;
+}
+
+// log2(threads / 128) per ROI: CTAs of 128 threads when several ROIs share an SM anyway, wider ones when the ROIs
+// do not fill the GPU and a ROI's latency decides (8 lanes per QI radius at most, so 8 nr threads). 50 ROIs of
+// 128x128 u8: 36 us with 512 threads each, 76 us with 128 and the tile as floats. 256 threads for every count cost
+// 4-8 % where several ROIs share an SM (1,000 x 64x64, 10,000 x 100x100).
+static int wide_cta(const TrackParams &P, int count)
+{
+    if (packed_rows(P.width, P.tile_pitch)) return 0;  // its COM's order depends on the thread count
+    const int per_sm = (count + 147) / 148;
+    if (per_sm <= 1 && P.qi_nr >= 64) return 2;
+    if (per_sm <= 2 && P.qi_nr >= 32) return 1;
+    return 0;
 }
 
 static bool g_attrs_set[64];
@@ -456,16 +552,19 @@ cudaError_t prepare_kernels(int device)
 {
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     if (g_attrs_set[device]) return cudaSuccess;
-    const int max_smem = 227 * 1024;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(localize_qi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)))
+    for (int f = 0; f < 3; f++)
+        for (int t = 0; t < 3; t++) {
+            if ((e = cudaFuncSetAttribute(reinterpret_cast<const void *>(kQiKernels[f][t]),
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)))
+                return e;
+            if ((e = cudaFuncSetAttribute(reinterpret_cast<const void *>(kLutKernels[f][t]),
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)))
+                return e;
+        }
+    if ((e = cudaFuncSetAttribute(localize_gauss_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)))
         return e;
-    if ((e = cudaFuncSetAttribute(localize_qi_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)))
-        return e;
-    if ((e = cudaFuncSetAttribute(localize_gauss_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem)))
-        return e;
-    if ((e = cudaFuncSetAttribute(build_lut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem))) return e;
-    if ((e = cudaFuncSetAttribute(profile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem))) return e;
+    if ((e = cudaFuncSetAttribute(profile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem))) return e;
     if ((e = prepare_gauss_kernels())) return e;
     g_attrs_set[device] = true;
     return cudaSuccess;
@@ -484,18 +583,9 @@ cudaError_t launch_localize(const TrackParams &P, const uint8_t *pixels, int pit
         localize_gauss_kernel<<<count, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, roi_stride,
                                                                               roi_offsets, jobs, count, results);
     } else {
-        // bulk-copy staging: ROIs back to back at a 16-byte aligned stride, and a pixel count for
-        // which the copy size and the in-place offset (4 - bpp) n are whole 16-byte units
-        const int bpp = P.pdt == 0 ? 1 : (P.pdt == 1 ? 2 : 4);
-        const int n = P.width * P.height;
-        const bool staged = !roi_offsets && pitch == P.width * bpp && !(reinterpret_cast<uintptr_t>(pixels) & 15) &&
-                            !(roi_stride & 15) && !(n & 15);
-        if (staged)
-            localize_qi_kernel<true><<<count, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, roi_stride,
-                                                                                    roi_offsets, jobs, count, results);
-        else
-            localize_qi_kernel<false><<<count, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, roi_stride,
-                                                                                     roi_offsets, jobs, count, results);
+        const int wide = wide_cta(P, count);
+        kQiKernels[tile_format(P)][wide]<<<count, kBlockThreads << wide, P.smem_bytes, stream>>>(
+            P, pixels, pitch, roi_stride, roi_offsets, jobs, count, results);
     }
     return cudaGetLastError();
 }
@@ -580,10 +670,12 @@ void localize_node(const TrackParams &P, int count, cudaKernelNodeParams &kp)
     if (use_gauss_warp(P)) {
         gauss_warp_node(P, count, kp);
     } else {
-        kp.func = (P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI) ? reinterpret_cast<void *>(localize_gauss_kernel)
-                                                                   : reinterpret_cast<void *>(localize_qi_kernel<false>);
+        const bool gauss = (P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI);
+        const int wide = gauss ? 0 : wide_cta(P, count);
+        kp.func = gauss ? reinterpret_cast<void *>(localize_gauss_kernel)
+                        : reinterpret_cast<void *>(kQiKernels[tile_format(P)][wide]);
         kp.gridDim = dim3(count);
-        kp.blockDim = dim3(kBlockThreads);
+        kp.blockDim = dim3(kBlockThreads << wide);
         kp.sharedMemBytes = P.smem_bytes;
     }
 }
@@ -592,8 +684,9 @@ cudaError_t launch_build_lut(const TrackParams &P, const uint8_t *pixels, int pi
                              const float2 *known_pos, bool normalize, float *lut, cudaStream_t stream)
 {
     if (nbeads <= 0) return cudaSuccess;
-    build_lut_kernel<<<nbeads, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, nbeads, plane, known_pos,
-                                                                      normalize ? 1 : 0, lut);
+    const int wide = wide_cta(P, nbeads);
+    kLutKernels[tile_format(P)][wide]<<<nbeads, kBlockThreads << wide, P.smem_bytes, stream>>>(
+        P, pixels, pitch, nbeads, plane, known_pos, normalize ? 1 : 0, lut);
     return cudaGetLastError();
 }
 

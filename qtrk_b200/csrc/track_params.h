@@ -17,9 +17,9 @@ struct float2_host { float x, y; };
 namespace qtrk {
 
 constexpr int kMaxQIIterations = 32;
-// Threads per localization CTA (one ROI per CTA). Four warps: with a 100x100 float tile (45 KB of
-// shared memory) five CTAs fit on an SM, and the one-warp sections of each ROI (QI transform and
-// fits, Z fit) leave three warps idle rather than seven.
+// Threads per localization CTA (one ROI per CTA) when there are enough ROIs to fill the SMs. Four warps:
+// with a 100x100 tile (45 KB of shared memory) five CTAs fit on an SM, and the one-warp sections of each
+// ROI (QI transform and fits, Z fit) leave three warps idle rather than seven.
 constexpr int kBlockThreads = 128;
 
 // Mode bits (cputrack/qtrk_c_api.h:5-20 plus the library's extension bits).
@@ -85,7 +85,8 @@ struct TrackParams {
     float offset_factor, gain_factor;
 
     // Dynamic shared-memory layout (byte offsets), filled by the host
-    int sm_img, sm_tables, sm_work, sm_red, sm_misc, smem_bytes;
+    int sm_img, sm_tables, sm_zdirs, sm_work, sm_red, sm_misc, smem_bytes;
+    int tile_pitch;  // words per tile row
     unsigned *err_flag;  // mapped host word: |= 4 when a staged ROI copy did not arrive in time (QI kernel)
 };
 

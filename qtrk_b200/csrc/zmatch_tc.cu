@@ -20,7 +20,7 @@
 // LT_B200_ZMatchTF32 the operands are w p and w L rounded to TF32 (kind::tf32, K = 8 per MMA,
 // one MMA per K step) and d_k = 2^-9 (1.02) |p'| |L'_k| (kBoundScaleTF32). Threads
 // record those candidate planes from their TMEM rows; warps then compute the exact scores with
-// the plain path's per-plane function (zlut_score: one lane per plane, bins in order), take the
+// the plain path's per-plane function (zlut_score, one lane per plane), take the
 // argmax and run the 7-point fit (LsqQuadraticFit.h:132-176) with the plain path's warp code, so z
 // is the plain path's bit for bit.
 //
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kTileM, 1) zmatch_tc_kernel(ZMatchParams Q)
             int bk = -1;
             for (int i = lane; i < ncheck; i += 32) {
                 const int k = all ? i : s_cand[r * kMaxCand + i];
-                const double e = zlut_score(pr, lut + (size_t)k * nb, 1, Q.weights, nb);
+                const double e = zlut_score(pr, lut + (size_t)k * nb, Q.weights, nb, Q.planes);
                 if (e == e && (bk < 0 || e > best || (e == best && k < bk))) {
                     best = e;
                     bk = k;
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kTileM, 1) zmatch_tc_kernel(ZMatchParams Q)
             }
             if (bk < 0) bk = 0;
             const int s0 = max(bk - 3, 0), s1 = min(bk + 4, Q.planes);
-            if (lane < s1 - s0) win[lane] = zlut_score(pr, lut + (size_t)(s0 + lane) * nb, 1, Q.weights, nb);
+            if (lane < s1 - s0) win[lane] = zlut_score(pr, lut + (size_t)(s0 + lane) * nb, Q.weights, nb, Q.planes);
             __syncwarp();
             auto at = [&](int k) { return win[k - s0]; };
             const float zz = max_interp7_sym(at, Q.planes, bk, kZLUTWeightsTC);

@@ -1,0 +1,129 @@
+"""The localization kernel's tile: formats, alignments, CTA widths and layouts.
+
+Whatever way a ROI reaches the kernel, its result is the same bit for bit: the pixel sums, the COM's chains and
+the circles' direction subsets are cut alike in every form. Against the FP64 oracle the parity tests'
+tolerances hold (COM 1e-4 px, QI 1e-3 px, Z 0.01 plane).
+"""
+import numpy as np
+import pytest
+
+from qtrk_b200 import abi, synth
+from qtrk_b200.tracker import QTrkInstance, computed_config
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("pos", "firstGuess", "error", "imageMean")
+
+
+def beads(w, n, dtype, seed=3):
+    rng = np.random.Generator(np.random.PCG64(seed * 1000 + w))
+    cx, cy = w / 2 + rng.uniform(-0.03, 0.03, n) * w, w / 2 + rng.uniform(-0.03, 0.03, n) * w
+    bg, amp, top = (200.0, 2000.0, 4095) if dtype == np.uint16 else (20.0, 180.0, 255)
+    lam = synth.render(w, w, cx, cy, rng.uniform(0.1, 0.45, n) * w, bg, amp)
+    return np.minimum(rng.poisson(8 * lam) // 8, top).astype(dtype)
+
+
+def device_run(t, rois, offset=0, jobs=None):
+    """LocalizeDevice on a stack that starts `offset` pixels into its buffer."""
+    import torch
+
+    n, _, w = rois.shape
+    flat = np.zeros(offset + rois.size, rois.dtype)
+    flat[offset:] = rois.ravel()
+    d = torch.from_numpy(flat.view(np.uint8)).cuda()
+    out = torch.zeros(n * 52, dtype=torch.uint8, device="cuda")
+    b = rois.itemsize
+    t.LocalizeDevice(d.data_ptr() + offset * b, w * b, w * w * b, abi.NUMPY_PDT[rois.dtype], n, out.data_ptr(),
+                     stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return np.frombuffer(out.cpu().numpy().tobytes(), dtype=abi.RESULT_DTYPE)
+
+
+def same(a, b, note):
+    for f in FIELDS:
+        assert np.array_equal(a[f], b[f]), (note, f)
+
+
+def tracker(s, lut, mode=synth.MODE_QI_Z):
+    t = QTrkInstance(s)
+    t.SetRadialZLUT(lut)
+    t.SetLocalizationMode(mode)
+    return t
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+@pytest.mark.parametrize("w,bg", [(40, 0.0), (61, 0.5), (64, 0.0), (78, 0.0), (99, 0.5), (100, 0.0), (128, 0.5)])
+def test_every_form_gives_the_same_bits(w, bg, dtype):
+    n = 1200
+    few = beads(w, 40, dtype)
+    rois = np.ascontiguousarray(few[np.arange(n) % 40])
+    s = synth.settings_square(w, com_bgcorrection=bg)
+    cc = computed_config(s)
+    lut = np.random.default_rng(w).normal(size=(1, 60, cc.zlut_radialsteps)).astype(np.float32)
+    with tracker(s, lut) as t:
+        for clear in (0, abi.LT_ClearFirstFourPixels):
+            t.SetLocalizationMode(synth.MODE_QI_Z | clear)
+            ref = device_run(t, few[:1])                     # one CTA per SM at most: the widest form
+            many = device_run(t, rois)                       # several per SM: 128 threads
+            same(many[:1], ref, "count")
+            same(many[:40], device_run(t, few), "count 40")
+            same(many[:250], device_run(t, rois[:250]), "count 250")
+            same(many[:40], many[40:80], "repeat")
+            for off in (1, 3, 8):                            # unaligned stacks
+                same(many[:300], device_run(t, rois[:300], off), f"offset {off}")
+            if dtype != np.float32:                          # float tile of the same pixel values
+                same(many[:300], device_run(t, rois[:300].astype(np.float32)), "float")
+            # frame bands: ROIs cropped at odd positions (bead 0's LUT only for the first)
+            cols = 6
+            frame = np.zeros((7 * (w + 3), cols * (w + 1) + 1), dtype)
+            pos = [(1 + (k % cols) * (w + 1), (k // cols) * (w + 3)) for k in range(40)]
+            for k, (x, y) in enumerate(pos):
+                frame[y:y + w, x:x + w] = few[k]
+            assert t.ScheduleFrame(frame, np.array(pos, np.int32)) == 40
+            r = t.WaitForResults(40)
+            r = r[np.argsort(r["zlutIndex"])]
+            assert np.array_equal(r["pos"][:, :2], many["pos"][:40, :2])
+            for f in FIELDS[1:]:
+                if f != "error":
+                    assert np.array_equal(r[f], many[f][:40]), f
+            same(r[:1], many[:1], "frame")
+
+
+@pytest.mark.parametrize("w,dtype,radial,n", [
+    (24, np.uint8, 0.9, 12),                                  # 2 nr = 16: transform through shared memory
+    (37, np.uint16, 1.4, 12), (64, np.float32, 0.6, 12),      # 2 nr = 32
+    (75, np.uint8, 1.4, 12), (75, np.uint8, 1.4, 700),        # 64
+    (100, np.uint16, 1.4, 12), (100, np.uint16, 1.4, 700),    # 128
+    (101, np.float32, 2.6, 8),                                # 256
+    (64, np.uint16, 8.0, 8),                                  # 512
+    (64, np.uint8, 16.0, 6),                                  # 1024: shared memory again
+    (236, np.uint16, 1.4, 3), (237, np.uint8, 1.4, 3)])       # compact and packed shared-memory layouts
+def test_sizes_match_fp64(port, w, dtype, radial, n):
+    few = beads(w, min(n, 12), dtype, seed=5)
+    rois = np.ascontiguousarray(few[np.arange(n) % len(few)])
+    s = synth.settings_square(w, qi_radial_coverage=radial)
+    if w < 32:
+        s.qi_minradius = s.zlut_minradius = 1.0
+    cc = computed_config(s)
+    planes = 50
+    stack = synth.render(w, w, np.full(planes, w / 2), np.full(planes, w / 2), np.linspace(0.05, 0.5, planes) * w, 200.0,
+                         2000.0).astype(np.float32)
+    with QTrkInstance(s) as t:
+        t.SetRadialZLUTSize(1, planes)
+        t.BeginLUT(True)
+        for k in range(planes):
+            t.BuildLUT(stack[k][None], k, known_pos=np.array([[w / 2, w / 2]], np.float32))
+        t.FinalizeLUT()
+        lut = t.GetRadialZLUT()
+    want_lut = port.build_lut(cc, stack[:, None], 4, known_pos=np.array([[w / 2, w / 2]], np.float32))
+    assert np.abs(lut - want_lut).max() < 1e-4
+    with tracker(s, lut) as t:
+        r = device_run(t, rois)
+    want = port.localize(cc, synth.MODE_QI_Z, few, lut)
+    want = want[np.arange(n) % len(few)]
+    assert np.abs(r["firstGuess"] - want[:, 3:5]).max() < 1e-4
+    assert np.abs(r["pos"][:, :2] - want[:, :2]).max() < 1e-3
+    inside = (want[:, 2] > 1) & (want[:, 2] < planes - 2)
+    assert inside.any()
+    assert np.abs(r["pos"][inside, 2] - want[inside, 2]).max() < 0.01
+    assert np.abs(r["imageMean"] - want[:, 6]).max() < 1e-3
