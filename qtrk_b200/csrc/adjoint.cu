@@ -14,103 +14,186 @@
 // Profiles are recomputed from the ROI (kept in shared memory), never stored as polar samples.
 #include <cstdint>
 
-#include "device_common.cuh"
 #include "kernels.h"
+#include "tile.cuh"
 
 namespace qtrk {
 
 namespace {
 
-constexpr int kAdjThreads = 256;
+constexpr int kAdjThreads = 128;     // adjoint: eight CTAs per SM hide its one-warp section
+constexpr int kRefineThreads = 256;  // joint refinement: many profiles of one ROI in turn
+constexpr int kGaussNllThreads = 256;
 constexpr int kRefineSteps = 5;
 constexpr float kPriorScale = 100.0f;  // x, y prior stiffness / z curvature (see joint_refine_kernel)
 
-// Bilinear sample with its x and y derivatives inside the cell (same index rule as bilinear()).
-__device__ __forceinline__ bool bilinear_grad(const float *img, int w, int h, float x, float y, float &v, float &gx,
-                                              float &gy)
-{
-    if (!(x > -1.0f && x < (float)(w - 1) && y > -1.0f && y < (float)(h - 1))) return false;
-    const float kMagic = 8388608.0f;
-    const float tx = __fadd_rz(fmaxf(x, 0.0f), kMagic), ty = __fadd_rz(fmaxf(y, 0.0f), kMagic);
-    const int rx = __float_as_int(tx) - 0x4B000000, ry = __float_as_int(ty) - 0x4B000000;
-    const float *p = img + ry * w + rx;
-    const float v00 = p[0], v10 = p[1], v01 = p[w], v11 = p[w + 1];
-    const float fx = x - (tx - kMagic), fy = y - (ty - kMagic);
-    const float v0 = v00 + (v10 - v00) * fx;
-    const float v1 = v01 + (v11 - v01) * fx;
-    v = v0 + (v1 - v0) * fy;
-    gx = (v10 - v00) * (1.0f - fy) + (v11 - v01) * fy;
-    gy = v1 - v0;
-    return true;
-}
-
 struct AdjSmem {
-    float *img;          // [H][W]
-    double *p, *dx, *dy; // [nb] profile and its x/y derivatives (normalised in place)
-    double *red;         // 128 doubles of reduction scratch (BlockGroup::sum<4>)
-    double *misc;        // 16 doubles: broadcast values
+    uint32_t *img;        // the tile (tile.cuh)
+    double *p, *dx, *dy;  // [nb] profile and its x/y derivatives (normalised in place)
+    double *red;          // 32 doubles of reduction scratch
+    double *misc;         // 16 doubles: broadcast values, the last one the mbarrier of the ROI's copy
 };
 
-__host__ __device__ inline int adj_img_bytes(const TrackParams &P) { return ((P.width * P.height * 4) + 15) & ~15; }
-
-__host__ __device__ inline int adj_smem_bytes(const TrackParams &P)
+__host__ __device__ inline int adj_smem_bytes(const TrackParams &P, int ts)
 {
-    return adj_img_bytes(P) + 3 * P.z_nbins * 8 + 128 * 8 + 16 * 8;
+    return tile_region_bytes(P.width, P.height, ts) + 3 * P.z_nbins * 8 + 32 * 8 + 16 * 8;
 }
 
-__device__ AdjSmem adj_view(uint8_t *smem, const TrackParams &P)
+// Padded rows where they fit in shared memory.
+inline int adj_pitch(const TrackParams &P)
+{
+    const int ts = tile_pitch(P.width);
+    return adj_smem_bytes(P, ts) <= 227 * 1024 ? ts : P.width;
+}
+
+__device__ __forceinline__ AdjSmem adj_view(uint8_t *smem, const TrackParams &P, int ts)
 {
     AdjSmem s;
-    s.img = reinterpret_cast<float *>(smem);
-    double *d = reinterpret_cast<double *>(smem + adj_img_bytes(P));
+    s.img = reinterpret_cast<uint32_t *>(smem);
+    double *d = reinterpret_cast<double *>(smem + tile_region_bytes(P.width, P.height, ts));
     s.p = d;
     s.dx = d + P.z_nbins;
     s.dy = d + 2 * P.z_nbins;
     s.red = d + 3 * P.z_nbins;
-    s.misc = s.red + 128;
+    s.misc = s.red + 32;
     return s;
 }
 
-// Profile (and derivatives) at (cx, cy): warps over bins, lanes over directions; FP32 sums of the
-// <= ceil(angsteps / 32) samples of a lane, FP64 across lanes. Ends with a block barrier.
-__device__ void profile_grad(const float *img, const TrackParams &P, float cx, float cy, float mean, double *p,
-                             double *dx, double *dy)
+// Load the ROI's tile; every thread gets the image mean (FP64 sum; asked only where a bin falls back to it).
+template <int F, int T>
+__device__ __forceinline__ float adj_load(const AdjSmem &s, const TrackParams &P, int ts, const uint8_t *src, int pitch,
+                                          int bead)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int nb = P.z_nbins;
+    const int W = P.width, n = W * P.height;
+    uint32_t isum = 0u;
+    if (F == kTileF32 && packed_rows(W, ts)) {
+        load_roi(BlockGroup{s.red}, reinterpret_cast<float *>(s.img), src, pitch, P, bead);
+    } else {
+        const uint8_t *raw = load_raw<F, T>(s.img, ts, P, src, pitch, reinterpret_cast<uint64_t *>(s.misc + 15), [] {});
+        convert_raw<F, T>(s.img, raw, ts, P, bead, isum);
+    }
+    __syncthreads();
+    double v[1] = {(double)isum};  // integer pixels: exact
+    if (F == kTileF32) {
+        v[0] = 0.0;
+        const int units = ((W + 3) >> 2) * P.height;
+        UnitWalk w(threadIdx.x, T, W, ts);
+        for (int u = threadIdx.x; u < units; u += T, w.step())
+            for (int j = 0; j < 4 && w.x + j < W; j++) v[0] += (double)__uint_as_float(s.img[w.off + j]);
+    }
+    BlockGroup{s.red}.sum<1>(v);
+    return (float)(v[0] / n);
+}
+
+// Profile (and derivatives) at (cx, cy), ROI in the tile: as radial_profile, eight lanes per bin with the direction
+// pairs (j, j + h), j = lane, lane + 8, ..., two samples per step in packed FP32x2; four pairs are summed in FP32
+// and folded into FP64. The x-derivative of a sample is d0 (1 - fy) + d1 fy, its y-derivative v1 - v0 (the values
+// cells2 returns). Sample coordinates are fma(d, r, c), as before: which cell a sample near a pixel edge falls
+// into decides its derivative. Ends with a block barrier.
+template <int F, int T>
+__device__ __forceinline__ void profile_grad(const uint32_t *img, int ts, const TrackParams &P, float cx, float cy,
+                                             float mean, double *p, double *dx, double *dy)
+{
+    const int nb = P.z_nbins, W = P.width, H = P.height, sub = threadIdx.x & 7, h = P.z_angsteps >> 1;
+    const bool odd = (P.z_angsteps & 1) != 0;
     const float rstep = (P.z_maxr - P.z_minr) / (float)nb;
     const float2 *dirs = static_cast<const float2 *>(P.z_dirs);
-    for (int bin = warp; bin < nb; bin += nw) {
+    const TileAddr ta(img, ts);
+    const float2 K = make_float2(kBias, kBias), nK = make_float2(-kBias, -kBias), m1 = make_float2(-1.0f, -1.0f);
+    const float2 one = make_float2(1.0f, 1.0f);
+    const double inv_all = 1.0 / P.z_angsteps;
+#pragma unroll 1
+    for (int bin = threadIdx.x >> 3; bin - (int)((threadIdx.x & 31) >> 3) < nb; bin += T / 8) {
         const float r = P.z_minr + rstep * (float)bin;
-        float s = 0.0f, sx = 0.0f, sy = 0.0f;
+        double s = 0.0, sx = 0.0, sy = 0.0;
         int c = 0;
-        for (int a = lane; a < P.z_angsteps; a += 32) {
-            const float2 d = dirs[a];
-            float v, gx, gy;
-            if (bilinear_grad(img, P.width, P.height, cx + d.x * r, cy + d.y * r, v, gx, gy)) {
-                s += v;
-                sx += gx;
-                sy += gy;
-                c++;
+        // one path per warp
+        const bool inside = __all_sync(0xffffffffu, bin >= nb || circle_inside(cx, cy, fabsf(r), W, H));
+        const float2 rr = make_float2(r, r), cxx = make_float2(cx, cx), cyy = make_float2(cy, cy);
+        if (inside) {
+            float2 a = make_float2(0.0f, 0.0f), ax = a, ay = a;
+            auto fold = [&] {
+                s += (double)(a.x + a.y);
+                sx += (double)(ax.x + ax.y);
+                sy += (double)(ay.x + ay.y);
+                a = ax = ay = make_float2(0.0f, 0.0f);
+            };
+            auto pair = [&](float2 d0, float2 d1) {
+                const float2 X = __ffma2_rn(make_float2(d0.x, d1.x), rr, cxx);
+                const float2 Y = __ffma2_rn(make_float2(d0.y, d1.y), rr, cyy);
+                const float2 TX = __fadd2_rz(X, K), TY = __fadd2_rz(Y, K);
+                const float2 FX = __ffma2_rn(__fadd2_rn(TX, nK), m1, X), FY = __ffma2_rn(__fadd2_rn(TY, nK), m1, Y);
+                const Cells q = cells2<F>(ta.at(ta.row(TY.x), TX.x), ta.at(ta.row(TY.y), TX.y), ta.ts4);
+                const float2 v0 = __ffma2_rn(q.d0, FX, q.v00), v1 = __ffma2_rn(q.d1, FX, q.v01);
+                const float2 gy = __ffma2_rn(v0, m1, v1);
+                a = __fadd2_rn(a, __ffma2_rn(gy, FY, v0));
+                ay = __fadd2_rn(ay, gy);
+                ax = __fadd2_rn(ax, __ffma2_rn(q.d1, FY, __fmul2_rn(q.d0, __ffma2_rn(FY, m1, one))));
+            };
+            const int np = bin < nb && sub < h ? (h - sub + 7) >> 3 : 0;
+            const float2 *dl = dirs + sub;
+            int k = 0;
+#pragma unroll 1
+            for (; k + 2 <= np; k += 2) {
+                pair(__ldg(dl + 8 * k), __ldg(dl + 8 * k + h));
+                pair(__ldg(dl + 8 * k + 8), __ldg(dl + 8 * k + 8 + h));
+                if (k & 2) fold();
             }
-        }
-        double ds = s, dsx = sx, dsy = sy;
+            if (k < np) pair(__ldg(dl + 8 * k), __ldg(dl + 8 * k + h));
+            fold();
+            if (odd && sub == 0 && bin < nb) {
+                const float2 d = __ldg(dirs + P.z_angsteps - 1);
+                pair(d, d);
+                s += (double)a.x;
+                sx += (double)ax.x;
+                sy += (double)ay.x;
+            }
+            c = P.z_angsteps;
+        } else {
+            const float xhi = (float)(W - 1), yhi = (float)(H - 1);
+            const int end = bin < nb ? P.z_angsteps : 0;
+            float a = 0.0f, ax = 0.0f, ay = 0.0f;
+            int in_part = 0;
+#pragma unroll 1
+            for (int j = sub; j < end; j += 8) {
+                const float2 d = __ldg(dirs + j);
+                const float x = fmaf(d.x, r, cx), y = fmaf(d.y, r, cy);
+                if (x > -1.0f && x < xhi && y > -1.0f && y < yhi) {
+                    const float tx = __fadd_rz(fmaxf(x, 0.0f), kBias), ty = __fadd_rz(fmaxf(y, 0.0f), kBias);
+                    const float fx = x - (tx - kBias), fy = y - (ty - kBias);
+                    const uint32_t w = ta.at(ta.row(ty), tx);
+                    const Cells q = cells2<F>(w, w, ta.ts4);
+                    const float v0 = fmaf(q.d0.x, fx, q.v00.x), v1 = fmaf(q.d1.x, fx, q.v01.x);
+                    a += fmaf(v1 - v0, fy, v0);
+                    ax += fmaf(q.d1.x, fy, q.d0.x * (1.0f - fy));
+                    ay += v1 - v0;
+                    c++;
+                }
+                if (++in_part == 5) {  // FP32 partials of five samples
+                    s += (double)a;
+                    sx += (double)ax;
+                    sy += (double)ay;
+                    a = ax = ay = 0.0f;
+                    in_part = 0;
+                }
+            }
+            s += (double)a;
+            sx += (double)ax;
+            sy += (double)ay;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            ds += __shfl_xor_sync(0xffffffffu, ds, o);
-            dsx += __shfl_xor_sync(0xffffffffu, dsx, o);
-            dsy += __shfl_xor_sync(0xffffffffu, dsy, o);
-            c += __shfl_xor_sync(0xffffffffu, c, o);
+            for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
         }
-        if (lane == 0) {
-            if (c > 4) {
-                p[bin] = ds / c;
-                dx[bin] = dsx / c;
-                dy[bin] = dsy / c;
-            } else {
-                p[bin] = mean;
-                dx[bin] = dy[bin] = 0.0;
-            }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        }
+        if (sub == 0 && bin < nb) {
+            const double inv = inside ? inv_all : 1.0 / c;
+            p[bin] = c > 4 ? s * inv : (double)mean;
+            dx[bin] = c > 4 ? sx * inv : 0.0;
+            dy[bin] = c > 4 ? sy * inv : 0.0;
         }
     }
     __syncthreads();
@@ -134,31 +217,33 @@ struct CostTerms {
 __device__ CostTerms cost_terms(const TrackParams &P, double *p, double *dx, double *dy, const float *L, float z)
 {
     const int lane = threadIdx.x & 31, nb = P.z_nbins, planes = P.lut_planes;
+    __syncwarp();  // the sums below run as one warp
     if (P.mode & kLT_NormalizeProfile) {
+        const double inv_nb = 1.0 / nb;
         double m = 0, mx = 0, my = 0;
         for (int i = lane; i < nb; i += 32) {
             m += p[i];
             mx += dx[i];
             my += dy[i];
         }
-        m = warp_sum(m) / nb;
-        mx = warp_sum(mx) / nb;
-        my = warp_sum(my) / nb;
+        m = warp_sum(m) * inv_nb;
+        mx = warp_sum(mx) * inv_nb;
+        my = warp_sum(my) * inv_nb;
         double ss = 0;
         for (int i = lane; i < nb; i += 32) ss += (p[i] - m) * (p[i] - m);
-        const double rms = sqrt(warp_sum(ss) / nb);
+        const double inv_rms = 1.0 / sqrt(warp_sum(ss) * inv_nb);
         double kx = 0, ky = 0;
         for (int i = lane; i < nb; i += 32) {
-            const double ph = (p[i] - m) / rms;
+            const double ph = (p[i] - m) * inv_rms;
             p[i] = ph;
             kx += ph * dx[i];
             ky += ph * dy[i];
         }
-        kx = warp_sum(kx) / nb;
-        ky = warp_sum(ky) / nb;
+        kx = warp_sum(kx) * inv_nb;
+        ky = warp_sum(ky) * inv_nb;
         for (int i = lane; i < nb; i += 32) {
-            dx[i] = (dx[i] - mx - p[i] * kx) / rms;
-            dy[i] = (dy[i] - my - p[i] * ky) / rms;
+            dx[i] = (dx[i] - mx - p[i] * kx) * inv_rms;
+            dy[i] = (dy[i] - my - p[i] * ky) * inv_rms;
         }
     }
     int iz = (int)floorf(z);
@@ -186,35 +271,26 @@ __device__ CostTerms cost_terms(const TrackParams &P, double *p, double *dx, dou
     return t;
 }
 
-// Image mean of the ROI in shared memory (block-wide; every thread gets it).
-__device__ double roi_mean(const float *img, int n, double *red)
-{
-    double v[1] = {0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) v[0] += img[i];
-    BlockGroup{red}.sum<1>(v);
-    return v[0] / n;
-}
-
 // Adjoint: one block per ROI. xyz[3*roi], bead[roi] (or 0), out cost[roi], grad[3*roi], and
 // glut[bead][plane][bin] += dcost/dL (atomically: ROIs of a bead share its LUT rows).
-__global__ void __launch_bounds__(kAdjThreads) zcost_grad_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
-                                                                 int pitch, int64_t roi_stride, int count,
-                                                                 const float *__restrict__ xyz,
-                                                                 const int *__restrict__ beads, float *__restrict__ cost,
-                                                                 float *__restrict__ grad, float *__restrict__ glut)
+// What bounds it: instruction issue. A warp over the directions of one bin at a time, every sample checked and
+// scalar, took 25.4 k warp instructions per 80x80 ROI, the packed pairs and pixel formats 12.8 k: 51,200 ROIs of
+// 80x80 u16 with the LUT gradient 1.377 -> 0.79 ms.
+template <int F>
+__global__ void __launch_bounds__(kAdjThreads, 8)
+    zcost_grad_kernel(TrackParams P, int ts, const uint8_t *__restrict__ pixels, int pitch, int64_t roi_stride,
+                      int count, const float *__restrict__ xyz, const int *__restrict__ beads,
+                      float *__restrict__ cost, float *__restrict__ grad, float *__restrict__ glut)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     const int roi = blockIdx.x;
     if (roi >= count) return;
-    const AdjSmem s = adj_view(smem, P);
+    const AdjSmem s = adj_view(smem, P, ts);
     const int bead = beads ? beads[roi] : 0;
     const bool ok = bead >= 0 && bead < P.lut_count && P.lut_planes >= 2;
-    BlockGroup g{s.red};
-    load_roi(g, s.img, pixels + (int64_t)roi * roi_stride, pitch, P, ok ? bead : 0);
-    __syncthreads();
-    const double mean = roi_mean(s.img, P.width * P.height, s.red);
+    const float mean = adj_load<F, kAdjThreads>(s, P, ts, pixels + (int64_t)roi * roi_stride, pitch, ok ? bead : 0);
     const float x = xyz[3 * roi], y = xyz[3 * roi + 1], z = xyz[3 * roi + 2];
-    profile_grad(s.img, P, x, y, (float)mean, s.p, s.dx, s.dy);
+    profile_grad<F, kAdjThreads>(s.img, ts, P, x, y, mean, s.p, s.dx, s.dy);
     if (threadIdx.x >= 32) return;
     if (!ok) {
         if (threadIdx.x == 0) {
@@ -274,22 +350,20 @@ __device__ bool solve3(const double A6[6], const double rhs[3], double d[3])
 // 1e-9 x trace, Cramer's rule, and the step halved up to 4 times until the objective drops (the
 // refinement stops when none does); z is clamped to [0, planes-1]. The fallback value of sparse
 // bins is the ROI's image mean, as in the Z fit.
-__global__ void __launch_bounds__(kAdjThreads) joint_refine_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
-                                                                   int pitch, int64_t roi_stride,
-                                                                   const int64_t *__restrict__ roi_offsets,
-                                                                   const LocalizationJob *__restrict__ jobs, int count,
-                                                                   LocalizationResult *__restrict__ results)
+template <int F>
+__global__ void __launch_bounds__(kRefineThreads)
+    joint_refine_kernel(TrackParams P, int ts, const uint8_t *__restrict__ pixels, int pitch, int64_t roi_stride,
+                        const int64_t *__restrict__ roi_offsets, const LocalizationJob *__restrict__ jobs, int count,
+                        LocalizationResult *__restrict__ results)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     const int roi = blockIdx.x;
     if (roi >= count) return;
-    const AdjSmem s = adj_view(smem, P);
+    const AdjSmem s = adj_view(smem, P, ts);
     const int bead = jobs ? jobs[roi].zlutIndex : 0;
     if (bead < 0 || bead >= P.lut_count || P.lut_planes < 2) return;  // no LUT for this ROI: no Z fit to refine
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
-    BlockGroup g{s.red};
-    load_roi(g, s.img, pixels + off, pitch, P, bead);
-    __syncthreads();
+    adj_load<F, kRefineThreads>(s, P, ts, pixels + off, pitch, bead);
     LocalizationResult *res = results + roi;
     const float mean = res->imageMean;
     const float x0 = res->pos.x, y0 = res->pos.y;
@@ -298,7 +372,7 @@ __global__ void __launch_bounds__(kAdjThreads) joint_refine_kernel(TrackParams P
     const float *L = P.lut + (size_t)bead * planes * nb;
     double k = 0.0, cur = 0.0;
     for (int step = 0; step < kRefineSteps; step++) {
-        profile_grad(s.img, P, x, y, mean, s.p, s.dx, s.dy);
+        profile_grad<F, kRefineThreads>(s.img, ts, P, x, y, mean, s.p, s.dx, s.dy);
         if (threadIdx.x < 32) {
             const CostTerms t = cost_terms(P, s.p, s.dx, s.dy, L, z);
             if (threadIdx.x == 0) {
@@ -330,7 +404,7 @@ __global__ void __launch_bounds__(kAdjThreads) joint_refine_kernel(TrackParams P
             const double tstep = ldexp(1.0, -hv);
             const float nx = (float)(x + tstep * d0), ny = (float)(y + tstep * d1);
             const float nz = fminf(fmaxf((float)(z + tstep * d2), 0.0f), (float)(planes - 1));
-            profile_grad(s.img, P, nx, ny, mean, s.p, s.dx, s.dy);
+            profile_grad<F, kRefineThreads>(s.img, ts, P, nx, ny, mean, s.p, s.dx, s.dy);
             if (threadIdx.x < 32) {
                 const CostTerms t = cost_terms(P, s.p, s.dx, s.dy, L, nz);
                 if (threadIdx.x == 0)
@@ -359,7 +433,7 @@ __global__ void __launch_bounds__(kAdjThreads) joint_refine_kernel(TrackParams P
 // model (the model gauss5_mle fits, erff per column/row, FP32 per pixel, FP64 sums) and its
 // gradient sum (1 - I/mu) dmu/dp for p = (x, y, I0, bg, sigma) = params[5 roi ..]. One block per ROI;
 // windows of at most 32x32 pixels take gauss_nll_warp_kernel (gauss.cu).
-__global__ void __launch_bounds__(kAdjThreads) gauss_nll_grad_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
+__global__ void __launch_bounds__(kGaussNllThreads) gauss_nll_grad_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
                                                                      int pitch, int64_t roi_stride, int count,
                                                                      const float *__restrict__ params,
                                                                      float *__restrict__ nll, float *__restrict__ grad)
@@ -422,11 +496,12 @@ cudaError_t launch_zcost_grad(const TrackParams &P, const uint8_t *pixels, int p
                               cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
-    const int smem = adj_smem_bytes(P);
-    cudaError_t e = cudaFuncSetAttribute(zcost_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int ts = adj_pitch(P), smem = adj_smem_bytes(P, ts), f = tile_format(P, ts);
+    const auto kernel = f == kTileF32 ? zcost_grad_kernel<kTileF32>
+                                      : (f == kTileU16 ? zcost_grad_kernel<kTileU16> : zcost_grad_kernel<kTileU8>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    zcost_grad_kernel<<<count, kAdjThreads, smem, stream>>>(P, pixels, pitch, roi_stride, count, xyz, beads, cost, grad,
-                                                            glut);
+    kernel<<<count, kAdjThreads, smem, stream>>>(P, ts, pixels, pitch, roi_stride, count, xyz, beads, cost, grad, glut);
     return cudaGetLastError();
 }
 
@@ -439,7 +514,7 @@ cudaError_t launch_gauss_nll_grad(const TrackParams &P, const uint8_t *pixels, i
     const int smem = (int)((((size_t)((W * H + 3) & ~3) + 3 * (W + H)) * 4 + 15) / 16 * 16) + 6 * 32 * 8;
     cudaError_t e = cudaFuncSetAttribute(gauss_nll_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    gauss_nll_grad_kernel<<<count, kAdjThreads, smem, stream>>>(P, pixels, pitch, roi_stride, count, params, nll, grad);
+    gauss_nll_grad_kernel<<<count, kGaussNllThreads, smem, stream>>>(P, pixels, pitch, roi_stride, count, params, nll, grad);
     return cudaGetLastError();
 }
 
@@ -448,11 +523,12 @@ cudaError_t launch_joint_refine(const TrackParams &P, const uint8_t *pixels, int
                                 LocalizationResult *results, cudaStream_t stream)
 {
     if (count <= 0) return cudaSuccess;
-    const int smem = adj_smem_bytes(P);
-    cudaError_t e = cudaFuncSetAttribute(joint_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int ts = adj_pitch(P), smem = adj_smem_bytes(P, ts), f = tile_format(P, ts);
+    const auto kernel = f == kTileF32 ? joint_refine_kernel<kTileF32>
+                                      : (f == kTileU16 ? joint_refine_kernel<kTileU16> : joint_refine_kernel<kTileU8>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    joint_refine_kernel<<<count, kAdjThreads, smem, stream>>>(P, pixels, pitch, roi_stride, roi_offsets, jobs, count,
-                                                              results);
+    kernel<<<count, kRefineThreads, smem, stream>>>(P, ts, pixels, pitch, roi_stride, roi_offsets, jobs, count, results);
     return cudaGetLastError();
 }
 

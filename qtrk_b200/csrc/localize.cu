@@ -266,46 +266,24 @@ __device__ __forceinline__ float z_localize(const SmemView &s, const TrackParams
 // and 64 us); larger ROIs, five to an SM by their tiles, lose 1 % (10,000 of 100x100: 842 and 834 us).
 constexpr int kMinBlocks = 7;
 
-constexpr uint32_t kStageWaitLimit = 1u << 22;  // mbarrier polls before a staged copy counts as lost
-
-// Bring ROI bytes at `src` into the tile and measure mean and COM. A contiguous ROI arrives by one bulk copy
-// (cp.async.bulk, completion on an mbarrier) that thread 0 starts first, while the others fetch the tables;
-// its up to 15 bytes before and behind the whole 16-byte units are loaded directly. Frame bands, and
-// small or misaligned ROIs, are loaded row by row.
+// Bring the ROI at `src` into the tile and measure mean and COM; the tables are fetched under the copy.
 template <int F, int T>
 __device__ __forceinline__ ComResult load_tile(const SmemView &s, const TrackParams &P, const uint8_t *src, int pitch,
                                                int bead, float bgcorr)
 {
-    const int W = P.width, H = P.height, bpp = tile_bpp(P), bytes = W * H * bpp, ts = P.tile_pitch;
-    const int misalign = (int)(reinterpret_cast<uintptr_t>(src) & 15);
-    if (F == kTileF32 && packed_rows(W, ts)) {  // the largest odd ROIs: a tile without room for padded rows
+    const int W = P.width, H = P.height, ts = P.tile_pitch;
+    auto tables = [&] {
         load_qi_tables(s, P);
+        if (P.sm_zdirs != P.sm_tables) load_z_tables(s, P);
+    };
+    if (F == kTileF32 && packed_rows(W, ts)) {  // the largest odd ROIs: a tile without room for padded rows
+        tables();
         const BlockGroup g{s.red};
         float *img = reinterpret_cast<float *>(s.img);
         return com_from_sums(g, img, W, H, load_roi(g, img, src, pitch, P, bead), bgcorr);
     }
-    const bool bulk = pitch == W * bpp && bytes >= kMinBulkBytes && !(misalign & (bpp - 1));
-    uint8_t *raw = reinterpret_cast<uint8_t *>(s.img) + raw_offset(W, H, ts, bpp, bulk ? misalign : 0);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(s.misc) + 32);
-    if (bulk && threadIdx.x == 0) {
-        mbar_init(mbar);
-        bulk_load_inner(raw, src, bytes, mbar);
-    }
-    load_qi_tables(s, P);
-    if (P.sm_zdirs != P.sm_tables) load_z_tables(s, P);
-    if (bulk) {
-        load_ends(raw, src, bytes);
-        // one thread waits for the copy (its acquire, then the barrier, order the copied bytes
-        // before every thread's reads); the others wait at the barrier without polling
-        if (threadIdx.x == 0 && !mbar_wait(mbar, 0, kStageWaitLimit) && P.err_flag) atomicOr(P.err_flag, 4u);
-    } else {
-        load_rows<T>(raw, src, pitch, W * bpp, H);
-    }
-    __syncthreads();
-    if (F != kTileF32 && (P.mode & kLT_ClearFirstFourPixels)) {  // QueuedCPUTracker.cpp:280-282
-        if (threadIdx.x < 4 * bpp) raw[threadIdx.x] = 0;
-        __syncthreads();
-    }
+    const uint8_t *raw = load_raw<F, T>(s.img, ts, P, src, pitch, mbar, tables);
     uint32_t isum;
     const double sum = convert_raw<F, T>(s.img, raw, ts, P, bead, isum);
     return tile_com<F, T>(s.img, W, H, ts, sum, isum, bgcorr, s.red);
@@ -526,13 +504,6 @@ static const LutKernel kLutKernels[3][3] = {
     {build_lut_kernel<kTileU16, 128>, build_lut_kernel<kTileU16, 256>, build_lut_kernel<kTileU16, 512>},
     {build_lut_kernel<kTileU8, 128>, build_lut_kernel<kTileU8, 256>, build_lut_kernel<kTileU8, 512>}};
 
-// Integer pixels are packed unless calibration images turn them into fractions, or rows are.
-static int tile_format(const TrackParams &P)
-{
-    if (P.pdt == 2 || P.calib_count > 0 || packed_rows(P.width, P.tile_pitch)) return kTileF32;
-    return P.pdt == 1 ? kTileU16 : kTileU8;
-}
-
 // log2(threads / 128) per ROI: CTAs of 128 threads when several ROIs share an SM anyway, wider ones when the ROIs
 // do not fill the GPU and a ROI's latency decides (8 lanes per QI radius at most, so 8 nr threads). 50 ROIs of
 // 128x128 u8: 36 us with 512 threads each, 76 us with 128 and the tile as floats. 256 threads for every count cost
@@ -584,7 +555,7 @@ cudaError_t launch_localize(const TrackParams &P, const uint8_t *pixels, int pit
                                                                               roi_offsets, jobs, count, results);
     } else {
         const int wide = wide_cta(P, count);
-        kQiKernels[tile_format(P)][wide]<<<count, kBlockThreads << wide, P.smem_bytes, stream>>>(
+        kQiKernels[tile_format(P, P.tile_pitch)][wide]<<<count, kBlockThreads << wide, P.smem_bytes, stream>>>(
             P, pixels, pitch, roi_stride, roi_offsets, jobs, count, results);
     }
     return cudaGetLastError();
@@ -673,7 +644,7 @@ void localize_node(const TrackParams &P, int count, cudaKernelNodeParams &kp)
         const bool gauss = (P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI);
         const int wide = gauss ? 0 : wide_cta(P, count);
         kp.func = gauss ? reinterpret_cast<void *>(localize_gauss_kernel)
-                        : reinterpret_cast<void *>(kQiKernels[tile_format(P)][wide]);
+                        : reinterpret_cast<void *>(kQiKernels[tile_format(P, P.tile_pitch)][wide]);
         kp.gridDim = dim3(count);
         kp.blockDim = dim3(kBlockThreads << wide);
         kp.sharedMemBytes = P.smem_bytes;
@@ -685,7 +656,7 @@ cudaError_t launch_build_lut(const TrackParams &P, const uint8_t *pixels, int pi
 {
     if (nbeads <= 0) return cudaSuccess;
     const int wide = wide_cta(P, nbeads);
-    kLutKernels[tile_format(P)][wide]<<<nbeads, kBlockThreads << wide, P.smem_bytes, stream>>>(
+    kLutKernels[tile_format(P, P.tile_pitch)][wide]<<<nbeads, kBlockThreads << wide, P.smem_bytes, stream>>>(
         P, pixels, pitch, nbeads, plane, known_pos, normalize ? 1 : 0, lut);
     return cudaGetLastError();
 }

@@ -45,6 +45,13 @@ __host__ __device__ inline int raw_offset(int W, int H, int ts, int bpp, int mis
     return tile_region_bytes(W, H, ts) - ((W * H * bpp + 15) & ~15) - 16 + misalign;
 }
 
+// Integer pixels are packed unless calibration images turn them into fractions, or rows are.
+__host__ __device__ inline int tile_format(const TrackParams &P, int ts)
+{
+    if (P.pdt == 2 || P.calib_count > 0 || packed_rows(P.width, ts)) return kTileF32;
+    return P.pdt == 1 ? kTileU16 : kTileU8;
+}
+
 __host__ __device__ inline int tile_bpp(const TrackParams &P) { return P.pdt == 0 ? 1 : (P.pdt == 1 ? 2 : 4); }
 
 // ---- pixels of a word -----------------------------------------------------------------------------------
@@ -86,22 +93,24 @@ struct TileAddr {
     __device__ __forceinline__ uint32_t at(uint32_t row, float tx) const { return row + (__float_as_uint(tx) << 2); }
 };
 
-// Bilinear values of two samples whose cells start at the words at p and q, with fractions fx = (fx_p, fx_q) and
-// fy: v0 + (v1 - v0) fy with v0 = v00 + (v10 - v00) fx and v1 likewise from the row below, in packed FP32x2
-// (each component rounds as the scalar operation does; v10 - v00 is fma(v00, -1, v10), exact before its one
-// rounding).
+// The corners of two samples' cells, at the words at p and q: the upper and lower left pixels v00 and v01, and the
+// differences d0 = v10 - v00 and d1 = v11 - v01 along x (fma(v00, -1, v10), exact before its one rounding).
+struct Cells {
+    float2 v00, v01, d0, d1;
+};
+
 template <int F>
-__device__ __forceinline__ float2 cell2(uint32_t p, uint32_t q, uint32_t ts4, float2 fx, float2 fy)
+__device__ __forceinline__ Cells cells2(uint32_t p, uint32_t q, uint32_t ts4)
 {
     const float2 m1 = make_float2(-1.0f, -1.0f);
-    float2 v0, v1;
+    Cells c;
     if (F == kTileF32) {
-        const float2 v00 = make_float2(tile_float(p), tile_float(q)), v10 = make_float2(tile_float<4>(p), tile_float<4>(q));
+        c.v00 = make_float2(tile_float(p), tile_float(q));
+        c.d0 = __ffma2_rn(c.v00, m1, make_float2(tile_float<4>(p), tile_float<4>(q)));
         p += ts4;
         q += ts4;
-        const float2 v01 = make_float2(tile_float(p), tile_float(q)), v11 = make_float2(tile_float<4>(p), tile_float<4>(q));
-        v0 = __ffma2_rn(__ffma2_rn(v00, m1, v10), fx, v00);
-        v1 = __ffma2_rn(__ffma2_rn(v01, m1, v11), fx, v01);
+        c.v01 = make_float2(tile_float(p), tile_float(q));
+        c.d1 = __ffma2_rn(c.v01, m1, make_float2(tile_float<4>(p), tile_float<4>(q)));
     } else {
         const float2 nK = make_float2(-kBias, -kBias);
         const uint32_t p0 = tile_word(p), q0 = tile_word(q);
@@ -116,10 +125,23 @@ __device__ __forceinline__ float2 cell2(uint32_t p, uint32_t q, uint32_t ts4, fl
             b01 = make_float2(biased<F, 2>(p0), biased<F, 2>(q0));
             b11 = make_float2(biased<F, 3>(p0), biased<F, 3>(q0));
         }
-        v0 = __ffma2_rn(__ffma2_rn(b00, m1, b10), fx, __fadd2_rn(b00, nK));
-        v1 = __ffma2_rn(__ffma2_rn(b01, m1, b11), fx, __fadd2_rn(b01, nK));
+        c.d0 = __ffma2_rn(b00, m1, b10);
+        c.d1 = __ffma2_rn(b01, m1, b11);
+        c.v00 = __fadd2_rn(b00, nK);
+        c.v01 = __fadd2_rn(b01, nK);
     }
-    return __ffma2_rn(__ffma2_rn(v0, m1, v1), fy, v0);
+    return c;
+}
+
+// Bilinear values of the two samples with fractions fx = (fx_p, fx_q) and fy: v0 + (v1 - v0) fy with
+// v0 = v00 + (v10 - v00) fx and v1 likewise from the row below, in packed FP32x2 (each component rounds as the
+// scalar operation does).
+template <int F>
+__device__ __forceinline__ float2 cell2(uint32_t p, uint32_t q, uint32_t ts4, float2 fx, float2 fy)
+{
+    const Cells c = cells2<F>(p, q, ts4);
+    const float2 v0 = __ffma2_rn(c.d0, fx, c.v00), v1 = __ffma2_rn(c.d1, fx, c.v01);
+    return __ffma2_rn(__ffma2_rn(v0, make_float2(-1.0f, -1.0f), v1), fy, v0);
 }
 
 // The same for one sample.
@@ -216,6 +238,41 @@ struct SmallDiv {
     __device__ __forceinline__ explicit SmallDiv(int d) : inv(1.0f / (float)d) {}
     __device__ __forceinline__ int operator()(int i) const { return (int)(((float)i + 0.5f) * inv); }
 };
+
+constexpr uint32_t kStageWaitLimit = 1u << 22;  // mbarrier polls before a staged copy counts as lost
+
+// Bring the ROI at `src` to the raw area of the tile region and return where it starts. A contiguous ROI arrives by
+// one bulk copy (cp.async.bulk, completion on an mbarrier) that thread 0 starts first, while all run `meanwhile`
+// (fetching tables); its up to 15 bytes before and behind the whole 16-byte units are loaded directly. Frame
+// bands, and small or misaligned ROIs, are loaded row by row. Ends with a barrier.
+template <int F, int T, typename Fn>
+__device__ __forceinline__ const uint8_t *load_raw(uint32_t *tile, int ts, const TrackParams &P, const uint8_t *src,
+                                                   int pitch, uint64_t *mbar, const Fn &meanwhile)
+{
+    const int W = P.width, H = P.height, bpp = tile_bpp(P), bytes = W * H * bpp;
+    const int misalign = (int)(reinterpret_cast<uintptr_t>(src) & 15);
+    const bool bulk = pitch == W * bpp && bytes >= kMinBulkBytes && !(misalign & (bpp - 1));
+    uint8_t *raw = reinterpret_cast<uint8_t *>(tile) + raw_offset(W, H, ts, bpp, bulk ? misalign : 0);
+    if (bulk && threadIdx.x == 0) {
+        mbar_init(mbar);
+        bulk_load_inner(raw, src, bytes, mbar);
+    }
+    meanwhile();
+    if (bulk) {
+        load_ends(raw, src, bytes);
+        // one thread waits for the copy (its acquire, then the barrier, order the copied bytes
+        // before every thread's reads); the others wait at the barrier without polling
+        if (threadIdx.x == 0 && !mbar_wait(mbar, 0, kStageWaitLimit) && P.err_flag) atomicOr(P.err_flag, 4u);
+    } else {
+        load_rows<T>(raw, src, pitch, W * bpp, H);
+    }
+    __syncthreads();
+    if (F != kTileF32 && (P.mode & kLT_ClearFirstFourPixels)) {  // QueuedCPUTracker.cpp:280-282
+        if (threadIdx.x < 4 * bpp) raw[threadIdx.x] = 0;
+        __syncthreads();
+    }
+    return raw;
+}
 
 // Walks the tile's units at a fixed stride. A unit is four pixels of a row from a column that is a multiple of
 // four (the last of a row may reach past it): unit u is at row u / upr, column 4 (u mod upr), upr units per row.

@@ -127,3 +127,49 @@ def test_sizes_match_fp64(port, w, dtype, radial, n):
     assert inside.any()
     assert np.abs(r["pos"][inside, 2] - want[inside, 2]).max() < 0.01
     assert np.abs(r["imageMean"] - want[:, 6]).max() < 1e-3
+
+
+@pytest.mark.parametrize("w,dtype", [(48, np.uint8), (61, np.uint16), (75, np.uint8), (80, np.uint16), (81, np.float32),
+                                     (100, np.uint8), (237, np.uint16)])
+def test_cost_gradient_sizes_match_fp64(port, w, dtype):
+    """The adjoint over every tile format, whole and ragged rows, aligned and unaligned stacks, circles inside the
+    image and across its edge. FP32 samples: 2e-4 of the cost; a sample within rounding of a pixel edge may take
+    the neighbouring cell's derivative, one of a bin's samples in one bin: 5e-3 of the largest component."""
+    import torch
+
+    n = 10
+    rois = beads(w, n, dtype, seed=7)
+    s = synth.settings_square(w)
+    cc = computed_config(s)
+    rng = np.random.default_rng(w)
+    planes = 20
+    lut = rng.normal(size=(3, planes, cc.zlut_radialsteps)).astype(np.float32)
+    beads_of = (np.arange(n) % 3).astype(np.int32)
+    xyz = np.stack([w / 2 + rng.uniform(-1, 1, n), w / 2 + rng.uniform(-1, 1, n), rng.uniform(0, planes - 1, n)], 1)
+    xyz[-2:, :2] += w * 0.3  # circles leave the image
+    xyz = xyz.astype(np.float32)
+    with tracker(s, lut) as t:
+        outs = []
+        for off in (0, 3):
+            flat = np.zeros(off + rois.size, dtype)
+            flat[off:] = rois.ravel()
+            px, d = torch.from_numpy(flat.view(np.uint8)).cuda(), torch.from_numpy(xyz).cuda()
+            b = torch.from_numpy(beads_of).cuda()
+            cost, grad = torch.empty(n, device="cuda"), torch.empty(n, 3, device="cuda")
+            glut = torch.zeros(lut.shape, device="cuda")
+            k = rois.itemsize
+            assert t.lib.QTrkB200ZLUTCostGradient(t.handle, px.data_ptr() + off * k, w * k, w * w * k,
+                                                  abi.NUMPY_PDT[rois.dtype], n, d.data_ptr(), b.data_ptr(),
+                                                  cost.data_ptr(), grad.data_ptr(), glut.data_ptr(), None) == 0
+            torch.cuda.synchronize()
+            outs.append([v.cpu().numpy().astype(np.float64) for v in (cost, grad, glut)])
+    assert np.array_equal(outs[0][0], outs[1][0]) and np.array_equal(outs[0][1], outs[1][1])
+    cost, grad, glut = outs[0]
+    want_l = np.zeros(lut.shape)
+    for i, img in enumerate(rois.astype(np.float64)):
+        c, g, gl = port.zcost_grad(img, img.mean(), xyz[i].astype(np.float64), lut[beads_of[i]], cc.zlut_angularsteps,
+                                   s.zlut_minradius, cc.zlut_maxradius, want_lut_grad=True)
+        want_l[beads_of[i]] += gl
+        assert abs(cost[i] - c) < 2e-4 * c
+        assert np.abs(grad[i] - g).max() < 5e-3 * np.abs(g).max()
+    assert np.abs(glut - want_l).max() < 2e-3 * np.abs(want_l).max()
