@@ -511,7 +511,8 @@ static const LutKernel kLutKernels[3][3] = {
 static int wide_cta(const TrackParams &P, int count)
 {
     if (packed_rows(P.width, P.tile_pitch)) return 0;  // its COM's order depends on the thread count
-    const int per_sm = (count + 147) / 148;
+    // ROIs that share an SM: by their number, or as many as its shared memory holds
+    const int per_sm = std::min((count + 147) / 148, (228 * 1024) / (P.smem_bytes + 1024));
     if (per_sm <= 1 && P.qi_nr >= 64) return 2;
     if (per_sm <= 2 && P.qi_nr >= 32) return 1;
     return 0;
