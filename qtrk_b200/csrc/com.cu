@@ -5,7 +5,9 @@
 //   v' = max(0, |v - mean| - bgcorrection * stdev),  COM = (sum x v', sum y v') / sum v'.
 // The fused localization kernel stages every ROI as a float tile in shared memory because QI and
 // the radial profile sample it many times; a COM-only localization reads each pixel twice and
-// needs no tile. Three forms, by ROI size:
+// needs no tile. Four forms, by ROI size:
+//  - com_column_kernel (ROIs of at least 8 columns in whole 4-pixel units, no background threshold): as
+//    com_warp_kernel, with a fixed column of units per thread;
 //  - com_warp_kernel (ROIs up to 55 KB): a group of 2-4 warps per ROI and one shared-memory buffer
 //    per group, filled by a bulk copy; both passes run over the raw buffer and the sums meet
 //    through warp shuffles and a named barrier per group, with no CTA-wide barrier;
@@ -21,6 +23,7 @@
 // sum x v' = x0 S + Sj - W Sw and sum y v' = y0 S + Sw, so each pixel costs two adds and one
 // multiply-add on top of the background correction, and only chunks that cross a row end pay
 // for Sw.
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 
@@ -588,6 +591,183 @@ __global__ void __launch_bounds__(1024, 1) com_warp_kernel(TrackParams P, const 
     }
 }
 
+// The column form of com_warp_kernel, for W a multiple of 4 and no background threshold: thread t of a group holds
+// the unit (four pixels) of column 4 (t mod W/4) in rows r0, r0 + R, ... (R = T / (W/4) rows per step; the threads
+// past R whole rows idle). With its column fixed a thread needs no chunk walk and no row-end split, and x
+// leaves the sums: sum x v' = x0 sum v' + sum j v'. Four steps at a time: a block's row sums S_k give sum S_k and
+// sum k S_k with constant factors. FP32 sums of at most 32 pixels meet in FP64; integer pixels are summed
+// exactly for the mean.
+// What bounds it: instruction issue. Per 8 pixels pass 2 takes about 40 instructions (load, unpacking, |v - mean|,
+// sums) where the walk over 16-byte chunks took 53: 10,000 x 100x100 u16 55.8 -> 46.9 us (65 % of the measured copy
+// rate, 54 % before), 8,000 x 100x100 f32 72.4 -> 52.8 us (92 %).
+template <int PDT>
+__global__ void __launch_bounds__(640, 2) com_column_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
+                                                             int64_t roi_stride, const LocalizationJob *__restrict__ jobs,
+                                                             int count, LocalizationResult *__restrict__ results,
+                                                             int buf_stride, int wg)
+{
+    constexpr int bpp = PDT == 0 ? 1 : (PDT == 1 ? 2 : 4);
+    extern __shared__ __align__(128) uint8_t bufs[];
+    __shared__ uint64_t mbar[kComMaxGroups];
+    __shared__ double red1[kComMaxGroups][4];
+    __shared__ double red2[kComMaxGroups][4][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = warp / wg, r = warp - grp * wg, ngrp = (blockDim.x >> 5) / wg;
+    const int T = 32 * wg, t = 32 * r + lane, bar_id = 1 + grp;
+    const bool leader = t == 0;
+    const int W = P.width, H = P.height, n = W * H, cpr = W >> 2, R = T / cpr;
+    const int r0 = t / cpr, x0 = 4 * (t - r0 * cpr);
+    const int steps = r0 < R ? (H - r0 + R - 1) / R : 0;
+    const uint32_t bytes = (uint32_t)(n * bpp);
+    uint8_t *gbuf = bufs + (size_t)grp * buf_stride;
+    const uint8_t *first = gbuf + (r0 * W + x0) * bpp;
+    const int rstep = R * W * bpp;
+    uint64_t *mb = &mbar[grp];
+    const int stride = gridDim.x * ngrp;
+    int roi = blockIdx.x * ngrp + grp;
+    if (leader) {
+        mbar_init(mb);
+        if (roi < count) bulk_load(gbuf, pixels + (int64_t)roi * roi_stride, bytes, mb);
+    }
+    const bool clear4 = (P.mode & kLT_ClearFirstFourPixels) != 0;
+    const float invN = 1.0f / (float)n;
+    for (uint32_t it = 0; roi < count; roi += stride, it++) {
+        // as in com_warp_kernel: wait, clear, pass the outcome to the group
+        const bool ok = leader ? mbar_wait(mb, it & 1u, kComWaitLimit) : true;
+        if (leader && ok && clear4)
+            for (int k = 0; k < bpp; k++) reinterpret_cast<uint32_t *>(gbuf)[k] = 0u;
+        if (!group_all(ok, bar_id, T)) {
+            if (leader) {
+                if (P.err_flag) atomicOr(P.err_flag, 4u);
+                mbar_wait(mb, it & 1u, kComWaitLimit);
+            }
+            return;
+        }
+        __syncwarp();
+        // pass 1
+        double m1 = 0.0;
+        {
+            const uint8_t *p = first;
+            if (PDT != 2) {
+                uint32_t si = 0u;  // exact: a ROI here has less than 2^16 pixels
+#pragma unroll 4
+                for (int k = 0; k < steps; k++, p += rstep) {
+                    if (PDT == 0) {
+                        si = __dp4a(*reinterpret_cast<const uint32_t *>(p), 0x01010101u, si);
+                    } else {
+                        const uint2 q = *reinterpret_cast<const uint2 *>(p);
+                        si = __dp2a_lo(q.x, 0x0101u, si);
+                        si = __dp2a_lo(q.y, 0x0101u, si);
+                    }
+                }
+                m1 = (double)__reduce_add_sync(0xffffffffu, si);
+            } else {
+                for (int k = 0; k < steps;) {
+                    float s = 0.0f;
+                    for (const int end = min(steps, k + 8); k < end; k++, p += rstep) {
+                        const float4 q = *reinterpret_cast<const float4 *>(p);
+                        s += (q.x + q.y) + (q.z + q.w);
+                    }
+                    m1 += (double)s;
+                }
+                m1 = warp_sum(m1);
+            }
+        }
+        if (lane == 0) red1[grp][r] = m1;
+        group_sync(bar_id, T);
+        m1 = 0.0;
+        for (int k = 0; k < wg; k++) m1 += red1[grp][k];
+        const float mean = (float)(m1 * (double)invN);
+        // pass 2: S = sum v' of a unit, Sj = sum j v'
+        const float2 nK = make_float2(-8388608.0f, -8388608.0f), nm = make_float2(-mean, -mean);
+        auto unit = [&](const uint8_t *p, float &S, float &Sj) {
+            float2 a, b;
+            if (PDT == 2) {
+                const float4 q = *reinterpret_cast<const float4 *>(p);
+                a = make_float2(q.x, q.y);
+                b = make_float2(q.z, q.w);
+            } else if (PDT == 1) {
+                const uint2 q = *reinterpret_cast<const uint2 *>(p);
+                a = make_float2(__uint_as_float(__byte_perm(q.x, 0x4B000000u, 0x7410u)),
+                                __uint_as_float(__byte_perm(q.x, 0x4B000000u, 0x7432u)));
+                b = make_float2(__uint_as_float(__byte_perm(q.y, 0x4B000000u, 0x7410u)),
+                                __uint_as_float(__byte_perm(q.y, 0x4B000000u, 0x7432u)));
+            } else {
+                const uint32_t q = *reinterpret_cast<const uint32_t *>(p);
+                a = make_float2(__uint_as_float(__byte_perm(q, 0x4B000000u, 0x7540u)),
+                                __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7541u)));
+                b = make_float2(__uint_as_float(__byte_perm(q, 0x4B000000u, 0x7542u)),
+                                __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7543u)));
+            }
+            if (PDT != 2) {
+                a = __fadd2_rn(a, nK);
+                b = __fadd2_rn(b, nK);
+            }
+            a = __fadd2_rn(a, nm);
+            b = __fadd2_rn(b, nm);
+            const float s23 = fabsf(b.x) + fabsf(b.y);
+            S = (fabsf(a.x) + fabsf(a.y)) + s23;
+            Sj = fmaf(2.0f, s23, fabsf(a.y) + fabsf(b.y));  // a1 + 2 a2 + 3 a3
+        };
+        double m2[3] = {0.0, 0.0, 0.0};
+        const uint8_t *p = first;
+        int k = 0;
+        float fy = (float)r0;
+        const float fR = (float)R;
+        while (k + 4 <= steps) {
+            float q0 = 0.0f, qj = 0.0f, qy = 0.0f;  // up to 8 steps, 32 pixels
+#pragma unroll 1
+            for (int h = 0; h < 2 && k + 4 <= steps; h++, k += 4, p += 4 * rstep) {
+                float S[4], Sj[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) unit(p + u * rstep, S[u], Sj[u]);
+                const float S4 = (S[0] + S[1]) + (S[2] + S[3]);
+                const float K4 = fmaf(3.0f, S[3], fmaf(2.0f, S[2], S[1]));
+                q0 += S4;
+                qj += (Sj[0] + Sj[1]) + (Sj[2] + Sj[3]);
+                qy += fmaf(fy, S4, fR * K4);
+                fy = fmaf(4.0f, fR, fy);
+            }
+            m2[0] += (double)q0;
+            m2[1] += (double)qj;
+            m2[2] += (double)qy;
+        }
+        if (k < steps) {
+            float q0 = 0.0f, qj = 0.0f, qy = 0.0f;
+#pragma unroll 1
+            for (; k < steps; k++, p += rstep, fy += fR) {
+                float S, Sj;
+                unit(p, S, Sj);
+                q0 += S;
+                qj += Sj;
+                qy = fmaf(fy, S, qy);
+            }
+            m2[0] += (double)q0;
+            m2[1] += (double)qj;
+            m2[2] += (double)qy;
+        }
+        m2[1] = fma((double)x0, m2[0], m2[1]);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 3; q++) m2[q] = warp_sum(m2[q]);
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < 3; q++) red2[grp][r][q] = m2[q];
+        // after this barrier every thread of the group has finished reading the buffer, so the
+        // leader may start the next copy into it
+        group_sync(bar_id, T);
+        if (leader) {
+            const int next = roi + stride;
+            if (next < count) bulk_load(gbuf, pixels + (int64_t)next * roi_stride, bytes, mb);
+            double m[3] = {0.0, 0.0, 0.0};
+            for (int q = 0; q < wg; q++)
+#pragma unroll
+                for (int v = 0; v < 3; v++) m[v] += red2[grp][q][v];
+            com_result(results, roi, jobs, m, mean, W, H);
+        }
+    }
+}
+
 namespace {
 
 using ComWarpKernel = void (*)(TrackParams, const uint8_t *, int64_t, const LocalizationJob *, int,
@@ -604,6 +784,46 @@ bool com_warp_plan(int64_t roi_bytes, int &groups, int &wg, int &stride)
     wg = 4;
     while (wg > 1 && groups * wg > 32) wg >>= 1;
     return groups >= 4;
+}
+
+// Buffers per CTA and warps per ROI (1, 2 or 4) of the column form. A ROI costs `work` warp steps (rows rounded up to
+// whole steps of R = T / (W/4) rows: 100 columns keep 125 of 128 threads busy, 50 of 64) and about six steps of
+// reductions per warp, and below about 18 warps per SM nothing hides the latencies (sweep of 12 to 160 px with 1,
+// 2 and 4 warps: 64 px u16 39.9, 41.3, 51.9 us; 80 px 48.3, 39.7, 47.9; 100 px 46.2, 45.7, 41.7; 128 px 55.8, 40.4,
+// 38.4). One CTA per SM or two (48 registers, at most 640 threads each), whichever keeps more ROIs in
+// flight. Integer rows of whole 8-pixel chunks cross no row end in com_warp_kernel, which is then the faster one
+// unless one or two warps fill at least 85 % of their lanes, 90 % for wide u8 rows (96 px u16: 40.9 us there,
+// 43.6 here; 112 px, 87.5 % of the lanes: u8 31.4 and 33.4, u16 47.2 and 42.7).
+bool com_column_plan(const TrackParams &P, int64_t roi_bytes, int &groups, int &wg, int &stride)
+{
+    const int cpr = P.width >> 2;
+    if ((P.width & 3) || P.width < 8 || cpr > 128 || P.com_bgcorrection != 0.0f) return false;
+    if ((int64_t)P.width * P.height >= 65536) return false;  // 32-bit pixel sums
+    stride = (int)((roi_bytes + 127) & ~(int64_t)127);
+    float best = 0.0f;
+    groups = 0;
+    bool full = false;
+    int in_flight = 0;
+    const int need = P.pdt == 0 && P.width > 64 ? 90 : 85;
+    for (int w = 1; w <= 4; w *= 2) {
+        const int R = 32 * w / cpr;
+        if (R < 1) continue;
+        if (w <= 2 && R * cpr * 100 >= need * 32 * w) full = true;
+        const int one = std::min({kComMaxGroups, (int)((220 * 1024) / stride), 20 / w});
+        const int two = std::min({kComMaxGroups, (int)((110 * 1024) / stride), 20 / w});
+        const int total = std::max(one, 2 * two), warps = total * w;
+        if (total < 1) continue;
+        const float work = (float)((P.height + R - 1) / R * w + 6 * w);
+        const float score = work * std::max(1.0f, 18.0f / (float)warps);
+        if (!groups || score < best) {
+            best = score;
+            wg = w;
+            groups = 2 * two >= one ? two : one;
+            in_flight = total;
+        }
+    }
+    if (P.pdt != 2 && !(P.width & 7) && !full) return false;
+    return in_flight >= 4;
 }
 
 using ComKernel = void (*)(TrackParams, const uint8_t *, int64_t, const LocalizationJob *, int, LocalizationResult *);
@@ -737,6 +957,17 @@ cudaError_t launch_com(const TrackParams &P, const uint8_t *pixels, int64_t roi_
     int stages = 0, stride = 0;
     const int64_t roi_bytes = (int64_t)P.width * P.height * bytes_per_pixel(P.pdt);
     int groups = 0, wg = 1;
+    if (com_column_plan(P, roi_bytes, groups, wg, stride)) {
+        ComWarpKernel f = P.pdt == 0 ? com_column_kernel<0> : (P.pdt == 1 ? com_column_kernel<1> : com_column_kernel<2>);
+        const int smem = groups * stride, threads = groups * wg * 32;
+        const int ctas = com_stream_ctas(reinterpret_cast<ComStreamKernel>(f), threads, smem);
+        if (ctas > 0) {
+            const int need = (count + groups - 1) / groups;
+            f<<<need < ctas ? need : ctas, threads, smem, stream>>>(P, pixels, roi_stride, jobs, count, results, stride,
+                                                                   wg);
+            return cudaGetLastError();
+        }
+    }
     if (com_warp_plan(roi_bytes, groups, wg, stride)) {
         ComWarpKernel f = P.pdt == 0 ? com_warp_kernel<0> : (P.pdt == 1 ? com_warp_kernel<1> : com_warp_kernel<2>);
         const int smem = groups * stride, threads = groups * wg * 32;

@@ -173,3 +173,32 @@ def test_cost_gradient_sizes_match_fp64(port, w, dtype):
         assert abs(cost[i] - c) < 2e-4 * c
         assert np.abs(grad[i] - g).max() < 5e-3 * np.abs(g).max()
     assert np.abs(glut - want_l).max() < 2e-3 * np.abs(want_l).max()
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+@pytest.mark.parametrize("w", [8, 12, 28, 36, 52, 56, 64, 76, 96, 100, 112, 116, 128, 160, 200])
+def test_com_only_sizes_match_fp64(w, dtype):
+    """LT_OnlyCOM over the widths that change its form, its warps per ROI and its ROIs in flight, with one ROI, a few
+    and more than the GPU holds at once. FP32 sums of at most 32 pixels: 2e-5 px; means of integers to one ulp."""
+    few = beads(w, 37, dtype, seed=9)
+    img = few.astype(np.float64)
+    s = synth.settings_square(w)
+    if w < 32:
+        s.qi_minradius = s.zlut_minradius = 0.25
+    for clear in (0, abi.LT_ClearFirstFourPixels):
+        if clear:
+            img[:, 0, :4] = 0
+        mean = img.mean((1, 2))
+        d = np.abs(img - mean[:, None, None])
+        at = np.arange(w)
+        want = np.stack([(d.sum(1) * at).sum(1), (d.sum(2) * at).sum(1)], 1) / d.sum((1, 2))[:, None]
+        with QTrkInstance(s) as t:
+            t.SetLocalizationMode(abi.LT_OnlyCOM | clear)
+            for n in (1, 7, 37, 3000 if w <= 128 else 400):
+                rois = np.ascontiguousarray(few[np.arange(n) % 37])
+                r = device_run(t, rois)
+                k = np.arange(n) % 37
+                assert np.abs(r["pos"][:, :2] - want[k]).max() < 2e-5
+                assert np.array_equal(r["pos"][:, :2], r["firstGuess"])
+                assert np.abs(r["imageMean"] - mean[k]).max() <= 2e-7 * mean.max() + 1e-7
+                assert np.array_equal(r["frame"], np.arange(n))
