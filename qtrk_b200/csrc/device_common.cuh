@@ -825,20 +825,22 @@ __device__ __forceinline__ double zlut_score(const float *prof, const float *lut
 // takes four planes (16-byte loads, four independent FP64 chains) over one run of bins. What a thread waits for
 // is the LUT (L2): one thread per plane over all bins in turn took 17.2 k of a 100x100 ROI's 146 k cycles (200 planes
 // x 64 bins, 128 threads, full load), this 7.1 k.
-template <bool kWeights>
+template <int T, bool kWeights>
 __device__ __forceinline__ void zlut_scores_runs(const float *prof, const float4 *lut4, int pitch4, int planes, int nb,
                                                  const float *weights, double *scores)
 {
     const int quads = (planes + 3) >> 2, lg = zlut_log2_runs(planes), len = (nb + (1 << lg) - 1) >> lg;
     const int total = quads << lg;
-    for (int base = 0; base < total; base += blockDim.x) {  // uniform: the sums below shuffle whole warps
+    // loads in flight per thread: more where one ROI has the SM to itself and waits for the LUT
+    constexpr int kUnroll = T >= 256 ? 8 : 4;
+    for (int base = 0; base < total; base += T) {  // uniform: the sums below shuffle whole warps
         const int t = base + threadIdx.x;
         if ((t & ~31) >= total) break;  // whole warps
         const int q = min(t >> lg, quads - 1), h = t & ((1 << lg) - 1);
         const int r0 = h * len, r1 = min(nb, r0 + len);
         const float4 *l = lut4 + (size_t)r0 * pitch4 + q;
         double v[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 4
+#pragma unroll kUnroll
         for (int r = r0; r < r1; r++, l += pitch4) {
             const float4 f = __ldg(l);
             const float p = prof[r];
@@ -861,14 +863,15 @@ __device__ __forceinline__ void zlut_scores_runs(const float *prof, const float4
     __syncthreads();
 }
 
+template <int T>
 __device__ __forceinline__ void zlut_scores_plain(const float *prof, const float *lut_t, int pitch, int planes, int nb,
                                                   const float *weights, double *scores)
 {
     const float4 *lut4 = reinterpret_cast<const float4 *>(lut_t);
     if (weights)
-        zlut_scores_runs<true>(prof, lut4, pitch >> 2, planes, nb, weights, scores);
+        zlut_scores_runs<T, true>(prof, lut4, pitch >> 2, planes, nb, weights, scores);
     else
-        zlut_scores_runs<false>(prof, lut4, pitch >> 2, planes, nb, weights, scores);
+        zlut_scores_runs<T, false>(prof, lut4, pitch >> 2, planes, nb, weights, scores);
 }
 
 // QueuedTracker::ZLUTBiasCorrection, cputrack/QueuedTracker.cpp:115-140: four fixed-point steps

@@ -74,11 +74,11 @@ __device__ __forceinline__ void fold_all(double *v, int lane, unsigned mask, int
     if constexpr (kO > 1) fold_all<H, kO / 2>(v, lane, mask, base, count);
 }
 
-// 1 / x to 1 ulp (one special-function instruction).
+// 1 / x to 1 ulp, subnormal x as zero (one special-function instruction).
 __device__ __forceinline__ float rcp(float x)
 {
     float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 

@@ -246,7 +246,7 @@ __device__ __forceinline__ float z_localize(const SmemView &s, const TrackParams
     if (!P.lut || bead < 0 || bead >= P.lut_count) return 0.0f;
     if (!P.lut_t) return __int_as_float(0x7fc00000);  // the host launched without refreshing the transposed LUT
     const float *lut_t = P.lut_t + (size_t)bead * nb * P.lut_t_pitch;
-    zlut_scores_plain(prof, lut_t, P.lut_t_pitch, P.lut_planes, nb, P.z_weights, scores);
+    zlut_scores_plain<T>(prof, lut_t, P.lut_t_pitch, P.lut_planes, nb, P.z_weights, scores);
     if (P.cmp_scores)
         for (int k = threadIdx.x; k < P.lut_planes; k += blockDim.x)
             P.cmp_scores[(size_t)bead * P.lut_planes + k] = (float)scores[k];
