@@ -905,6 +905,14 @@ __device__ __forceinline__ float zlut_bias_correct(float z, int planes, const fl
 // erf/exp terms depend only on the column (x) or the row (y), so they are evaluated once
 // per column and per row and combined per pixel.
 // -------------------------------------------------------------------------------------
+// 1 / x to 1 ulp, subnormal x as zero (one special-function instruction).
+__device__ __forceinline__ float rcp(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 __device__ __forceinline__ float erf_as(float x, float e_mx2)
 {
     // e_mx2 = exp(-x*x)
@@ -912,7 +920,7 @@ __device__ __forceinline__ float erf_as(float x, float e_mx2)
                 a5 = 1.061405429f, p = 0.3275911f;
     const float sign = x < 0 ? -1.0f : 1.0f;
     const float ax = fabsf(x);
-    const float t = 1.0f / (1.0f + p * ax);
+    const float t = rcp(1.0f + p * ax);
     const float y = 1.0f - (((((a5 * t + a4) * t) + a3) * t + a2) * t + a1) * t * e_mx2;
     return sign * y;
 }

@@ -15,7 +15,7 @@
 // is left per iteration: the sums across lanes, the divisions and the 5x5 solve.
 //
 // What bounds it: instruction issue (75 % used at 24-32 warps per SM). Measured on 100,000 16x16 f32
-// ROIs, 8 iterations: 4 parameters 1.520 -> 0.456 ms, 5 parameters (20,000 15x15 u16) 0.434 -> 0.145 ms
+// ROIs, 8 iterations: 4 parameters 1.520 -> 0.417 ms, 5 parameters (20,000 15x15 u16) 0.434 -> 0.137 ms
 // against one warp per ROI with every pixel forming all its products in FP32 and adding eight (or twenty)
 // sums; one warp per ROI with the column factors taken out reached 0.613 and 0.232 ms.
 #include <cstdint>
@@ -72,14 +72,6 @@ __device__ __forceinline__ void fold_all(double *v, int lane, unsigned mask, int
     base += up ? H : 0;
     count = up ? count - H : min(count, H);
     if constexpr (kO > 1) fold_all<H, kO / 2>(v, lane, mask, base, count);
-}
-
-// 1 / x to 1 ulp, subnormal x as zero (one special-function instruction).
-__device__ __forceinline__ float rcp(float x)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
 }
 
 // A symmetric definite 5x5 system (upper triangle in A, row by row) by elimination without pivoting,

@@ -273,6 +273,7 @@ Tracker::Tracker(const QTrkSettings &settings)
     CheckCuda(cudaEventCreateWithFlags(&lut_ready_, cudaEventDisableTiming), "cudaEventCreate");
     CheckCuda(cudaEventCreateWithFlags(&noalloc_order_, cudaEventDisableTiming), "cudaEventCreate");
     CheckCuda(cudaStreamCreateWithFlags(&lut_copy_stream_, cudaStreamNonBlocking), "cudaStreamCreate(lut copy)");
+    CheckCuda(cudaStreamCreateWithFlags(&frame_copy_stream_, cudaStreamNonBlocking), "cudaStreamCreate(frame copy)");
     for (int b = 0; b < 2; b++) {
         CheckCuda(cudaEventCreateWithFlags(&lut_stage_free_[b], cudaEventDisableTiming), "cudaEventCreate");
         CheckCuda(cudaEventCreateWithFlags(&lut_copy_done_[b], cudaEventDisableTiming), "cudaEventCreate");
@@ -294,6 +295,7 @@ Tracker::~Tracker()
         }
     }
     if (lut_stream_) cudaStreamSynchronize(lut_stream_);
+    if (frame_copy_stream_) cudaStreamSynchronize(frame_copy_stream_);
     for (Slot &s : slots_) {
         if (s.stream) cudaStreamSynchronize(s.stream);
         cudaFreeHost(s.h_pix);
@@ -303,7 +305,6 @@ Tracker::~Tracker()
         cudaFree(s.d_pix);
         cudaFree(s.d_jobs);
         cudaFree(s.d_res);
-        cudaFree(s.d_off);
         cudaFree(s.d_zprof);
         cudaFree(s.d_zprof_bf16);
         cudaFreeHost(s.h_perm);
@@ -340,6 +341,7 @@ Tracker::~Tracker()
     if (noalloc_order_) cudaEventDestroy(noalloc_order_);
     if (lut_stream_) cudaStreamDestroy(lut_stream_);
     if (lut_copy_stream_) cudaStreamDestroy(lut_copy_stream_);
+    if (frame_copy_stream_) cudaStreamDestroy(frame_copy_stream_);
 }
 
 TrackParams Tracker::Params(int pdt) const
@@ -684,7 +686,6 @@ void Tracker::AllocateSlots()
         CheckCuda(cudaHostAlloc(&sl.h_res, sizeof(LocalizationResult) * batch_, cudaHostAllocDefault), "cudaHostAlloc");
         CheckCuda(cudaMalloc(&sl.d_res, sizeof(LocalizationResult) * batch_), "cudaMalloc");
         CheckCuda(cudaHostAlloc(&sl.h_off, sizeof(int64_t) * batch_, cudaHostAllocDefault), "cudaHostAlloc");
-        CheckCuda(cudaMalloc(&sl.d_off, sizeof(int64_t) * batch_), "cudaMalloc");
         free_.push_back(i);
     }
 }
@@ -789,13 +790,15 @@ void Tracker::SubmitLocked(int idx)
         CheckCuda(cudaEventRecord(s.ev_start, s.stream), "cudaEventRecord");
         CheckCuda(cudaMemcpyAsync(s.d_pix, s.h_pix, roib * s.count, cudaMemcpyHostToDevice, s.stream), "H2D pixels");
     }
-    CheckCuda(cudaMemcpyAsync(s.d_jobs, s.h_jobs, sizeof(LocalizationJob) * s.count, cudaMemcpyHostToDevice, s.stream),
-              "H2D jobs");
-    if (s.frame)
-        CheckCuda(cudaMemcpyAsync(s.d_off, s.h_off, sizeof(int64_t) * s.count, cudaMemcpyHostToDevice, s.stream),
-                  "H2D offsets");
-    CheckCuda(launch_localize(P, s.d_pix, s.pitch, (int64_t)roib, s.frame ? s.d_off : nullptr, s.d_jobs, s.count,
-                              s.d_res, s.stream),
+    // A frame band's kernel reads its few bytes per ROI of jobs and offsets from pinned host memory: small copies
+    // between the bands' rows left the copy engine idle for about 15 us per band.
+    const LocalizationJob *jobs = s.frame ? s.h_jobs : s.d_jobs;
+    const int64_t *offsets = s.frame ? s.h_off : nullptr;
+    if (!s.frame)
+        CheckCuda(cudaMemcpyAsync(s.d_jobs, s.h_jobs, sizeof(LocalizationJob) * s.count, cudaMemcpyHostToDevice,
+                                  s.stream),
+                  "H2D jobs");
+    CheckCuda(launch_localize(P, s.d_pix, s.pitch, (int64_t)roib, offsets, jobs, s.count, s.d_res, s.stream),
               "localize kernel launch");
     launches_++;
     if (tc) {
@@ -810,8 +813,7 @@ void Tracker::SubmitLocked(int idx)
         launches_++;
     }
     if (RefineAfterZ(P)) {
-        CheckCuda(launch_joint_refine(P, s.d_pix, s.pitch, (int64_t)roib, s.frame ? s.d_off : nullptr, s.d_jobs,
-                                      s.count, s.d_res, s.stream),
+        CheckCuda(launch_joint_refine(P, s.d_pix, s.pitch, (int64_t)roib, offsets, jobs, s.count, s.d_res, s.stream),
                   "joint refine launch");
         launches_++;
     }
@@ -1041,11 +1043,12 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
     if (skipped) Warn("ScheduleFrame: skipped " + std::to_string(skipped) + " ROI(s) outside the frame");
     if (idx.empty()) return 0;
 
-    // Group ROIs into row bands of at most 32 MiB (or one slot, if smaller); one band keeps the
-    // caller's order. The bands' copies run one after another (each waits for the previous one),
+    // Group ROIs into row bands of at most 32 MiB (or one slot, if smaller); the bands of a frame listed in
+    // scan order keep the caller's order, and one band does. The bands' copies run one after another (each waits for the previous one),
     // so every band's kernel overlaps the next band's copy and only the last, small band's kernel
     // is left after the frame has crossed PCIe.
     const size_t band_cap = std::min(slot_bytes_, (size_t)32 << 20);
+    const bool pinned = IsPinned(img);
     int minx = width, maxx = 0;
     for (int i : idx) {
         minx = std::min(minx, pos[i].x);
@@ -1060,11 +1063,33 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
             y0 = std::min(y0, pos[i].y);
             y1 = std::max(y1, pos[i].y + H);
         }
+        auto by_row = [&](int a, int b) { return pos[a].y < pos[b].y; };
         if (span_bytes(y0, y1) <= band_cap && (int)idx.size() <= batch_) {
-            bands.push_back(idx);
+            // A frame of several megabytes crosses PCIe in up to three shrinking bands (3:2:1 of its rows), so that
+            // only the last, smallest band's kernel is left after the copy: 1,000 beads of 100x100 u16 in 20 MB,
+            // 582 us per frame in one band, 515 in three or four (the copy alone: 381). Rows that two bands
+            // share are copied twice: they may add at most a tenth. Only for frames listed in scan order,
+            // whose results then come in the same order.
+            int n = 1;
+            if (pinned && span_bytes(y0, y1) >= ((size_t)4 << 20) && std::is_sorted(idx.begin(), idx.end(), by_row))
+                for (n = std::min(3, (int)slots_.size()); n > 1; n--)
+                    if ((size_t)(n - 1) * H * dpitch * 10 <= span_bytes(y0, y1)) break;
+            std::vector<int> cur;
+            const int parts = n * (n + 1) / 2;
+            int part = n;  // share of the rows up to the current band's end
+            for (int i : idx) {
+                const int64_t end = (int64_t)(y1 - y0) * part / parts;
+                if (!cur.empty() && n > 1 && pos[i].y + H - y0 > end) {
+                    bands.push_back(cur);
+                    cur.clear();
+                    n--;
+                    part += n;
+                }
+                cur.push_back(i);
+            }
+            bands.push_back(cur);
         } else {
             std::vector<int> sorted = idx;
-            auto by_row = [&](int a, int b) { return pos[a].y < pos[b].y; };
             if (!std::is_sorted(sorted.begin(), sorted.end(), by_row))  // frames are usually listed in scan order
                 std::stable_sort(sorted.begin(), sorted.end(), by_row);
             std::vector<int> cur;
@@ -1103,7 +1128,6 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
         return count;
     }
 
-    const bool pinned = IsPinned(img);
     std::vector<cudaEvent_t> copies;  // one per band, in order: the copy chain
     std::unique_lock<std::mutex> lk(mu_);
     if (filling_ >= 0) {  // keep FIFO order with earlier single-ROI jobs
@@ -1137,14 +1161,15 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
             s.h_jobs[k].zlutIndex = i + job->zlutIndex;
         }
         CheckCuda(cudaEventRecord(s.ev_start, s.stream), "cudaEventRecord");
-        if (!copies.empty()) CheckCuda(cudaStreamWaitEvent(s.stream, copies.back(), 0), "cudaStreamWaitEvent");
+        // The bands' rows cross on one copy stream, back to back; only a band's kernel waits for them.
         const uint8_t *src = static_cast<const uint8_t *>(img) + (size_t)y0 * pitch + (size_t)minx * bpp;
         CheckCuda(cudaMemcpy2DAsync(s.d_pix, dpitch, src, (size_t)pitch, (size_t)(maxx - minx) * bpp, (size_t)(y1 - y0),
-                                    cudaMemcpyHostToDevice, s.stream),
+                                    cudaMemcpyHostToDevice, frame_copy_stream_),
                   "H2D frame rows");
         cudaEvent_t ev;
         CheckCuda(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate");
-        CheckCuda(cudaEventRecord(ev, s.stream), "cudaEventRecord");
+        CheckCuda(cudaEventRecord(ev, frame_copy_stream_), "cudaEventRecord");
+        CheckCuda(cudaStreamWaitEvent(s.stream, ev, 0), "cudaStreamWaitEvent");
         copies.push_back(ev);
         SubmitLocked(si);
         count += s.count;

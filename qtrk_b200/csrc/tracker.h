@@ -102,7 +102,7 @@ class Tracker : public QueuedTracker {
         uint8_t *h_pix = nullptr, *d_pix = nullptr;
         LocalizationJob *h_jobs = nullptr, *d_jobs = nullptr;
         LocalizationResult *h_res = nullptr, *d_res = nullptr;
-        int64_t *h_off = nullptr, *d_off = nullptr;
+        int64_t *h_off = nullptr;
         // tensor-core Z match scratch (allocated on first use): profiles between the two
         // kernels, the bead-grouped ROI order and the tile list
         float *d_zprof = nullptr;
@@ -110,7 +110,7 @@ class Tracker : public QueuedTracker {
         int *h_perm = nullptr, *d_perm = nullptr;
         int4 *h_tiles = nullptr, *d_tiles = nullptr;
         int count = 0, pdt = -1;
-        bool frame = false;   // pixels hold frame rows addressed through d_off
+        bool frame = false;   // pixels hold frame rows addressed through h_off
         int pitch = 0;
         double t_submit = 0;  // host seconds
     };
@@ -138,6 +138,7 @@ class Tracker : public QueuedTracker {
     int batch_ = 0;              // ROIs per slot
     size_t slot_bytes_ = 0;      // pixel bytes per slot
     std::vector<Slot> slots_;
+    cudaStream_t frame_copy_stream_ = nullptr;  // H2D of frame rows, all bands in order
     std::deque<int> free_, inflight_;
     int filling_ = -1;
 
