@@ -275,7 +275,7 @@ __device__ CostTerms cost_terms(const TrackParams &P, double *p, double *dx, dou
 // glut[bead][plane][bin] += dcost/dL (atomically: ROIs of a bead share its LUT rows).
 // What bounds it: instruction issue. A warp over the directions of one bin at a time, every sample checked and
 // scalar, took 25.4 k warp instructions per 80x80 ROI, the packed pairs and pixel formats 12.8 k: 51,200 ROIs of
-// 80x80 u16 with the LUT gradient 1.377 -> 0.79 ms.
+// 80x80 u16 with the LUT gradient 1.377 -> 0.76 ms.
 template <int F>
 __global__ void __launch_bounds__(kAdjThreads, 8)
     zcost_grad_kernel(TrackParams P, int ts, const uint8_t *__restrict__ pixels, int pitch, int64_t roi_stride,

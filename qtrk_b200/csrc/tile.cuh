@@ -7,11 +7,12 @@
 //   kTileU8   the pixel, its right, lower and lower right neighbours in the four bytes (u8 ROIs).
 // A bilinear sample needs the 2x2 pixels of its cell: four 32-bit shared loads of floats, two of pairs, one
 // of quads. As floats, 10,000 ROIs of 100x100 u16 kept the shared-memory pipe at 72 % (21.2 k wavefronts per ROI) and
-// issue at 50 %; as pairs they need 12.4 k, and what bounds the kernel is instruction issue (59 % used, 57 k
+// issue at 50 %; as pairs they need 12.4 k, and what bounds the kernel is instruction issue (61 % used, 59 k
 // warp instructions per ROI, a third of them the byte permutes and adds that turn packed pixels into floats)
 // with 20 warps per SM and one-warp sections (QI transform and fit) in between. Measured together with the
-// transform in registers, the LUT runs and the wider CTAs for few ROIs: 10,000 x 100x100 u16 1.002 -> 0.842 ms,
-// 1,000 x 64x64 u16 with own LUTs 127 -> 55 us, 50 x 128x128 u8 76 -> 36 us. All formats give bit-identical results for the same pixels: every later operation sees the same floats.
+// transform in registers, the LUT runs and the wider CTAs for few ROIs: 10,000 x 100x100 u16 1.002 -> 0.832 ms,
+// 1,000 x 64x64 u16 with own LUTs 127 -> 55 us, 50 x 128x128 u8 78 -> 35 us.
+// All formats give bit-identical results for the same pixels: every later operation sees the same floats.
 //
 // Results also do not depend on T (the launcher picks T by the number of ROIs): whatever is summed in FP32 is
 // cut into pieces that are the same for every T (the eight direction subsets of a circle, the 512 pixel
@@ -345,14 +346,15 @@ __device__ __forceinline__ void raw_five(const uint8_t *a, uint32_t &x, uint32_t
 // a batch overwrites no raw pixel of a later one. Returns this thread's pixel sum: exact as an integer
 // (isum), or FP32 sums of a unit's pixels added in FP64 (kTileF32). Every thread runs the same number of
 // batches.
-template <int F, int T>
-__device__ __forceinline__ double convert_raw(uint32_t *tile, const uint8_t *raw, int ts, const TrackParams &P, int bead,
-                                              uint32_t &isum)
+// kPlain: whole units that lie aligned in the raw ROI (read with one load) and, for kTileF32, are floats that nothing
+// changes; the other ROIs take a call.
+template <int F, int T, bool kPlain>
+__device__ __forceinline__ double convert_units(uint32_t *tile, const uint8_t *raw, int ts, const TrackParams &P,
+                                                int bead, uint32_t &isum)
 {
     const int W = P.width, H = P.height, n = W * H, upr = (W + 3) >> 2, units = upr * H;
-    const int bpp = F == kTileU16 ? 2 : (F == kTileU8 ? 1 : tile_bpp(P));
-    // whole units that lie aligned in the raw ROI are read with one load
-    const bool aligned = !(W & 3) && !((uint32_t)reinterpret_cast<uintptr_t>(raw) & (4 * bpp - 1));
+    const int bpp = F == kTileU16 ? 2 : (F == kTileU8 ? 1 : (kPlain ? 4 : tile_bpp(P)));
+    constexpr bool aligned = kPlain;
     double sum = 0.0;
     isum = 0u;
     UnitWalk w(threadIdx.x, T, W, ts);
@@ -427,11 +429,11 @@ __device__ __forceinline__ double convert_raw(uint32_t *tile, const uint8_t *raw
     } else {
         constexpr int kBatch = 4;
         const float *off = nullptr, *gain = nullptr;
-        if (bead >= 0 && bead < P.calib_count) {
+        if (!kPlain && bead >= 0 && bead < P.calib_count) {
             if (P.calib_offset) off = P.calib_offset + (size_t)bead * n;
             if (P.calib_gain) gain = P.calib_gain + (size_t)bead * n;
         }
-        const bool plain = !off && !gain && !(P.mode & kLT_ClearFirstFourPixels);
+        const bool plain = kPlain || (!off && !gain && !(P.mode & kLT_ClearFirstFourPixels));
 #pragma unroll 1
         for (int u0 = threadIdx.x, b0 = 0; b0 < units; b0 += kBatch * T, u0 += kBatch * T) {
             float f[kBatch][4];
@@ -439,7 +441,7 @@ __device__ __forceinline__ double convert_raw(uint32_t *tile, const uint8_t *raw
 #pragma unroll
             for (int k = 0; k < kBatch; k++) {
                 const int count = u0 + k * T < units ? min(4, W - v.x) : 0;
-                if (aligned && P.pdt == 2) {
+                if (aligned) {
                     const float4 q = count ? reinterpret_cast<const float4 *>(raw)[v.pix >> 2] : make_float4(0, 0, 0, 0);
                     f[k][0] = q.x, f[k][1] = q.y, f[k][2] = q.z, f[k][3] = q.w;
                 } else {
@@ -471,6 +473,49 @@ __device__ __forceinline__ double convert_raw(uint32_t *tile, const uint8_t *raw
             }
         }
     }
+    return sum;
+}
+
+// What the conversion of a ROI that is not plain needs of TrackParams (a call's arguments).
+struct RawForm {
+    int W, H, pdt, mode, calib_count;
+    float off_factor, gain_factor;
+    const float *offset, *gain;
+};
+
+template <int F, int T>
+__device__ __noinline__ double convert_call(uint32_t *tile, const uint8_t *raw, int ts, RawForm f, int bead,
+                                            uint32_t *isum)
+{
+    TrackParams P;
+    P.width = f.W;
+    P.height = f.H;
+    P.pdt = f.pdt;
+    P.mode = f.mode;
+    P.calib_count = f.calib_count;
+    P.calib_offset = f.offset;
+    P.calib_gain = f.gain;
+    P.offset_factor = f.off_factor;
+    P.gain_factor = f.gain_factor;
+    uint32_t s;
+    const double sum = convert_units<F, T, false>(tile, raw, ts, P, bead, s);
+    *isum = s;
+    return sum;
+}
+
+template <int F, int T>
+__device__ __forceinline__ double convert_raw(uint32_t *tile, const uint8_t *raw, int ts, const TrackParams &P, int bead,
+                                              uint32_t &isum)
+{
+    const int unit = 4 * (F == kTileU16 ? 2 : (F == kTileU8 ? 1 : 4));
+    bool plain = !(P.width & 3) && !((uint32_t)reinterpret_cast<uintptr_t>(raw) & (unit - 1));
+    if (F == kTileF32) plain = plain && P.pdt == 2 && P.calib_count == 0 && !(P.mode & kLT_ClearFirstFourPixels);
+    if (plain) return convert_units<F, T, true>(tile, raw, ts, P, bead, isum);
+    const RawForm f = {P.width,         P.height,       P.pdt,          P.mode,      P.calib_count,
+                       P.offset_factor, P.gain_factor, P.calib_offset, P.calib_gain};
+    uint32_t s;
+    const double sum = convert_call<F, T>(tile, raw, ts, f, bead, &s);
+    isum = s;
     return sum;
 }
 
@@ -569,6 +614,18 @@ __device__ __forceinline__ void com_moments(const uint32_t *tile, int W, int H, 
     }
 }
 
+// With a threshold, as a call: the kernels are fetched cold by small launches, and what few ROIs need stays out of
+// the way (with the conversions above: 10,000 100x100 u16 ROIs 0.846 -> 0.832 ms, the adjoint of 51,200 80x80 u16
+// ones 0.795 -> 0.763 ms).
+template <int F, int T>
+__device__ __noinline__ void com_moments_call(const uint32_t *tile, int W, int H, int ts, float mean, float thr,
+                                              double *m)
+{
+    double v[3] = {0.0, 0.0, 0.0};
+    com_moments<F, T, true>(tile, W, H, ts, mean, thr, v);
+    for (int k = 0; k < 3; k++) m[k] = v[k];
+}
+
 template <int F, int T>
 __device__ __forceinline__ ComResult tile_com(const uint32_t *tile, int W, int H, int ts, double sum, uint32_t isum,
                                               float bgcorr, double *red)
@@ -603,7 +660,7 @@ __device__ __forceinline__ ComResult tile_com(const uint32_t *tile, int W, int H
     }
     double m[3] = {0.0, 0.0, 0.0};
     if (bgcorr != 0.0f)
-        com_moments<F, T, true>(tile, W, H, ts, r.mean, thr, m);
+        com_moments_call<F, T>(tile, W, H, ts, r.mean, thr, m);
     else
         com_moments<F, T, false>(tile, W, H, ts, r.mean, 0.0f, m);
     g.sum(m);
