@@ -15,7 +15,7 @@
 // is left per iteration: the sums across lanes, the divisions and the 5x5 solve.
 //
 // What bounds it: instruction issue (75 % used at 24-32 warps per SM). Measured on 100,000 16x16 f32
-// ROIs, 8 iterations: 4 parameters 1.520 -> 0.417 ms, 5 parameters (20,000 15x15 u16) 0.434 -> 0.137 ms
+// ROIs, 8 iterations: 4 parameters 1.520 -> 0.403 ms, 5 parameters (20,000 15x15 u16) 0.434 -> 0.137 ms
 // against one warp per ROI with every pixel forming all its products in FP32 and adding eight (or twenty)
 // sums; one warp per ROI with the column factors taken out reached 0.613 and 0.232 ms.
 #include <cstdint>

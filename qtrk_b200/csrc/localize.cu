@@ -263,7 +263,7 @@ __device__ __forceinline__ float z_localize(const SmemView &s, const TrackParams
 
 // CTAs per SM the 128-thread kernels are compiled for (72 registers): ROIs of up to about 80 px fit seven times,
 // and a frame of 1,000 then runs in one wave (60x60 f32: 57 us, 70 us with five CTAs of 96 registers; 64x64 u16: 55
-// and 64 us); larger ROIs, five to an SM by their tiles, lose 1 % (10,000 of 100x100: 842 and 834 us).
+// and 64 us); larger ROIs, five to an SM by their tiles, lose 1 % by it.
 constexpr int kMinBlocks = 7;
 
 // Bring the ROI at `src` into the tile and measure mean and COM; the tables are fetched under the copy.
@@ -470,14 +470,15 @@ static void plan_smem_form(TrackParams &P, bool compact)
     const int nr = P.qi_nr > 0 ? P.qi_nr : 1, L = 2 * nr;
     P.sm_img = 0;
     P.tile_pitch = compact ? W : tile_pitch(W);
-    P.sm_tables = tile_region_bytes(W, H, P.tile_pitch);
+    // The CTA of the Gaussian modes loads row by row, so its compact form needs no room behind the tile for a raw ROI.
+    const bool gauss = (P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI);
+    P.sm_tables = compact && gauss ? align16(W * H * 4) : tile_region_bytes(W, H, P.tile_pitch);
     const int qi_tables = align16(P.qi_angpq * 16 + nr * 8 + nr * 4), z_tables = ((P.z_angsteps + 1) >> 1) * 16;
     P.sm_zdirs = compact ? P.sm_tables : P.sm_tables + qi_tables;
     P.sm_work = compact ? P.sm_tables + std::max(qi_tables, z_tables) : P.sm_zdirs + z_tables;
     // QI: the profile (L complex), and its transform where that runs through shared memory
     const int qi_work = (L >= 32 && L <= 512 ? 1 : 2) * L * 8;
     const int z_work = align16(P.z_nbins * 4) + P.lut_planes * 8;
-    const bool gauss = (P.mode & kLT_Gaussian2D) != 0;
     const int g_work = gauss ? (3 * W + 3 * H) * 4 : 0;
     P.sm_red = P.sm_work + align16(std::max(qi_work, std::max(z_work, g_work)));
     // block sum scratch, N * warps doubles: N <= 20 with 4 warps (Gaussian), 3 with up to 16
@@ -656,9 +657,12 @@ cudaError_t launch_build_lut(const TrackParams &P, const uint8_t *pixels, int pi
                              const float2 *known_pos, bool normalize, float *lut, cudaStream_t stream)
 {
     if (nbeads <= 0) return cudaSuccess;
-    const int wide = wide_cta(P, nbeads);
-    kLutKernels[tile_format(P, P.tile_pitch)][wide]<<<nbeads, kBlockThreads << wide, P.smem_bytes, stream>>>(
-        P, pixels, pitch, nbeads, plane, known_pos, normalize ? 1 : 0, lut);
+    TrackParams Q = P;  // the layout of a ROI that arrives raw, whatever the instance's mode
+    Q.mode &= ~kLT_Gaussian2D;
+    plan_smem(Q);
+    const int wide = wide_cta(Q, nbeads);
+    kLutKernels[tile_format(Q, Q.tile_pitch)][wide]<<<nbeads, kBlockThreads << wide, Q.smem_bytes, stream>>>(
+        Q, pixels, pitch, nbeads, plane, known_pos, normalize ? 1 : 0, lut);
     return cudaGetLastError();
 }
 

@@ -86,3 +86,33 @@ def test_gauss_nll_gradient_window_sizes_match_fp64(port, w, h):
             for k in range(5):
                 scale = max(1.0, abs(prm[i, 2]) if k in (0, 1, 4) else float(w * h if k == 3 else 1.0))
                 assert abs(float(grad[i, k]) - g[k]) < 1e-5 * scale + 1e-5 * abs(g[k]), (i, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(234, 234), (235, 235), (236, 234)])
+def test_gauss_windows_at_the_shared_memory_limit(port, w, h):
+    """Windows that fit only in the compact layout, whose Gaussian form leaves no room for a raw ROI: fits against
+    the FP64 oracle (FP32 terms over 55,000 pixels: 1e-3 px, the bound of QI positions), and a LUT built in that
+    mode, whose ROIs do arrive raw, equal to the one built in a QI mode."""
+    n, iters = 2, 14
+    rois, sigma = spots(w, h, n, np.uint16, w + 3 * h)
+    s = abi.settings(width=w, height=h, gauss2D_sigma=sigma, gauss2D_iterations=iters)
+    luts = []
+    for mode in (abi.LT_Gaussian2D, abi.LT_QI):
+        with QTrkInstance(s) as t:
+            t.SetLocalizationMode(mode)
+            if mode == abi.LT_Gaussian2D:
+                r = t.Localize(rois)
+            t.SetRadialZLUTSize(n, 2)
+            t.BeginLUT(abi.BUILDLUT_NORMALIZE)
+            for plane in range(2):
+                t.BuildLUT(rois, plane)
+            t.FinalizeLUT()
+            luts.append(t.GetRadialZLUT())
+    assert np.isfinite(luts[0]).all() and np.abs(luts[0]).max() > 0
+    np.testing.assert_array_equal(luts[0], luts[1])
+    for i in range(n):
+        img = rois[i].astype(np.float64)
+        com = port.com(img)
+        want = np.asarray(port.gauss2d(img, com[2], com[:2], iters, sigma))
+        assert np.abs(r["pos"][i, :2] - want[:2]).max() < 1e-3
