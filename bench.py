@@ -666,8 +666,8 @@ COM_BYTES_PER_ROI = 100 * 100 * 2 + 52  # pixels in, result out (no job records:
 
 
 def com_only_bench(dev, settings, d_rois, n: int, steps: int, warmup: int, sm_mhz: float | None = None) -> dict:
-    """LT_OnlyCOM on the headline stack (n ROIs of 100x100 u16 resident in HBM): the warp-per-ROI
-    COM kernel (bulk-copied ROI buffers, shuffle reductions), one launch per step, with its roofline
+    """LT_OnlyCOM on the headline stack (n ROIs of 100x100 u16 resident in HBM): the COM
+    column kernel (bulk-copied ROI buffers, a column of pixels per lane), one launch per step, with its roofline
     against the measured HBM copy rate."""
     import torch
 
@@ -685,7 +685,7 @@ def com_only_bench(dev, settings, d_rois, n: int, steps: int, warmup: int, sm_mh
     peaks, peak_kind = measured_peaks()
     achieved = COM_BYTES_PER_ROI * n / (ms / 1e3) / 1e9
     traffic = None
-    tfile = ROOT / "profiles" / "com_100x100_u16_traffic.json"
+    tfile = ROOT / "profiles" / "com_column_100x100_u16_traffic.json"
     if tfile.exists():
         traffic = json.loads(tfile.read_text()).get("dram_bytes_per_launch")
     roof_extra = issue_limits(tfile, ms, sm_mhz)
@@ -693,7 +693,7 @@ def com_only_bench(dev, settings, d_rois, n: int, steps: int, warmup: int, sm_mh
             "rois_per_s": n / (ms / 1e3), "ms_per_launch": ms, "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "qtrk::com_warp_kernel<1>", "kernel_ms": ms,
+                         "kernel": "qtrk::com_column_kernel<1>", "kernel_ms": ms,
                          "bytes_per_roi": COM_BYTES_PER_ROI, **roof_extra}}
 
 
@@ -1102,12 +1102,12 @@ def main(argv=None) -> int:
     peaks, peak_kind = measured_peaks()
     achieved = BYTES_PER_ROI * N_ROIS / (kernel_ms / 1e3) / 1e9
     traffic = None
-    tfile = ROOT / "profiles" / "localize_100x100_u16_traffic.json"
+    tfile = ROOT / "profiles" / "localize_pairs_100x100_u16_traffic.json"
     if tfile.exists():
         traffic = json.loads(tfile.read_text()).get("dram_bytes_per_launch")
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"], "traffic": traffic, "peak_kind": peak_kind,
-                "kernel": "qtrk::localize_qi_kernel<true>", "kernel_ms": kernel_ms,
+                "kernel": "qtrk::localize_qi_kernel<1, 128>", "kernel_ms": kernel_ms,
                 "bytes_per_roi": BYTES_PER_ROI}
     roofline.update(issue_limits(tfile, kernel_ms, clocks.get("sm_mhz")))
 
