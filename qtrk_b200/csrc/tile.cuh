@@ -67,8 +67,9 @@ __device__ __forceinline__ float biased(uint32_t w)
 
 constexpr float kBias = 8388608.0f;  // 2^23
 
-// A tile word at a 32-bit shared-memory address (+ kOff bytes). Not volatile: the tile does not change once it is
-// converted, and every sample's address depends on the COM taken behind the barrier that follows.
+// A tile word at a 32-bit shared-memory address (+ kOff bytes). Not volatile, so that loads of one sample may be
+// scheduled among another's arithmetic: the compiler sees a function of the address alone. What keeps it behind the
+// barrier that completes the tile is its address, which only a TileAddr gives.
 template <int kOff = 0>
 __device__ __forceinline__ uint32_t tile_word(uint32_t a)
 {
@@ -84,11 +85,15 @@ __device__ __forceinline__ float tile_float(uint32_t a)
 
 // Addresses of cells from biased coordinates (2^23 + the truncated coordinate, as the round-toward-zero add
 // leaves them): row() of a y and at() of an x in that row. The biases are folded into one constant.
+// Constructed behind the barrier that completes the tile. The base passes through a statement that the compiler keeps
+// in order with barriers and memory accesses, so that no address, and no load, exists before it: neither the
+// position nor the directions need to come from behind the barrier (the adjoint's come from global memory).
 struct TileAddr {
     uint32_t base, ts4;
     __device__ __forceinline__ TileAddr(const uint32_t *tile, int ts) : ts4(4u * ts)
     {
         base = smem_addr(tile) - 0x4B000000u * (ts4 + 4u);
+        asm volatile("" : "+r"(base)::"memory");
     }
     __device__ __forceinline__ uint32_t row(float ty) const { return __float_as_uint(ty) * ts4 + base; }
     __device__ __forceinline__ uint32_t at(uint32_t row, float tx) const { return row + (__float_as_uint(tx) << 2); }
