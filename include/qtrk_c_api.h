@@ -413,6 +413,11 @@ QTRK_API void QTRK_CALLCONV QTrkB200BuildLUTAsync(struct QueuedTracker *qtrk, vo
  * the latest instance), as the LabVIEW layer needs them. */
 QTRK_API void QTRK_CALLCONV QTrkB200SetPixelCalibrationFactors(struct QueuedTracker *qtrk, float offsetFactor,
                                                                float gainFactor);
+/* How often a kernel polls for a ROI's staged copy into shared memory before it gives the ROI up (default
+ * 4194304; following calls of this instance, LT_OnlyCOM excepted). A ROI given up is reported as a warning
+ * and is not a number: its result, its cost and gradients (the LUT's gradient gets nothing from it), its
+ * row in QTrkBuildLUT. */
+QTRK_API void QTRK_CALLCONV QTrkB200SetCopyWaitLimit(struct QueuedTracker *qtrk, uint32_t polls);
 QTRK_API void QTRK_CALLCONV QTrkB200EnableRadialZLUTCompareProfile(struct QueuedTracker *qtrk, int enable);
 QTRK_API void QTRK_CALLCONV QTrkB200GetRadialZLUTCompareProfile(struct QueuedTracker *qtrk, float *dst);
 /* SetCUDADevices (cudatrack/QueuedCUDATracker.cu): the device list for cuda_device = QTrkCUDA_UseList.

@@ -826,6 +826,11 @@ QTRK_API void QTRK_CALLCONV QTrkB200SetPixelCalibrationFactors(QueuedTracker *q,
             [&](Tracker *t) { t->SetPixelCalibrationFactors(offsetFactor, gainFactor); });
 }
 
+QTRK_API void QTRK_CALLCONV QTrkB200SetCopyWaitLimit(QueuedTracker *q, uint32_t polls)
+{
+    guarded(q, "QTrkB200SetCopyWaitLimit", [&](Tracker *t) { t->SetCopyWaitLimit(polls); });
+}
+
 QTRK_API void QTRK_CALLCONV QTrkB200EnableRadialZLUTCompareProfile(QueuedTracker *q, int enable)
 {
     guarded(q, "QTrkB200EnableRadialZLUTCompareProfile", [&](Tracker *t) { t->EnableRadialZLUTCompareProfile(enable != 0); });

@@ -245,12 +245,14 @@ struct SmallDiv {
     __device__ __forceinline__ int operator()(int i) const { return (int)(((float)i + 0.5f) * inv); }
 };
 
-constexpr uint32_t kStageWaitLimit = 1u << 22;  // mbarrier polls before a staged copy counts as lost
+constexpr uint32_t kStageWaitLimit = 1u << 22;  // mbarrier polls that a late copy gets before its CTA ends
 
 // Bring the ROI at `src` to the raw area of the tile region and return where it starts. A contiguous ROI arrives by
 // one bulk copy (cp.async.bulk, completion on an mbarrier) that thread 0 starts first, while all run `meanwhile`
 // (fetching tables); its up to 15 bytes before and behind the whole 16-byte units are loaded directly. Frame
 // bands, and small or misaligned ROIs, are loaded row by row. Ends with a barrier.
+// A copy that is late (P.copy_polls) is flagged and given a last bounded wait, since it writes into this CTA's shared
+// memory, and every thread gets nullptr: the caller writes NaN results and ends, with no word of the tile read.
 template <int F, int T, typename Fn>
 __device__ __forceinline__ const uint8_t *load_raw(uint32_t *tile, int ts, const TrackParams &P, const uint8_t *src,
                                                    int pitch, uint64_t *mbar, const Fn &meanwhile)
@@ -268,11 +270,17 @@ __device__ __forceinline__ const uint8_t *load_raw(uint32_t *tile, int ts, const
         load_ends(raw, src, bytes);
         // one thread waits for the copy (its acquire, then the barrier, order the copied bytes
         // before every thread's reads); the others wait at the barrier without polling
-        if (threadIdx.x == 0 && !mbar_wait(mbar, 0, kStageWaitLimit) && P.err_flag) atomicOr(P.err_flag, 4u);
+        bool arrived = true;
+        if (threadIdx.x == 0 && !mbar_wait(mbar, 0, P.copy_polls)) {
+            if (P.err_flag) atomicOr(P.err_flag, 4u);
+            mbar_wait(mbar, 0, kStageWaitLimit);
+            arrived = false;
+        }
+        if (!__syncthreads_and(arrived)) return nullptr;
     } else {
         load_rows<T>(raw, src, pitch, W * bpp, H);
+        __syncthreads();
     }
-    __syncthreads();
     if (F != kTileF32 && (P.mode & kLT_ClearFirstFourPixels)) {  // QueuedCPUTracker.cpp:280-282
         if (threadIdx.x < 4 * bpp) raw[threadIdx.x] = 0;
         __syncthreads();

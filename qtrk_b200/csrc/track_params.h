@@ -87,7 +87,8 @@ struct TrackParams {
     // Dynamic shared-memory layout (byte offsets), filled by the host
     int sm_img, sm_tables, sm_zdirs, sm_work, sm_red, sm_misc, smem_bytes;
     int tile_pitch;  // words per tile row
-    unsigned *err_flag;  // mapped host word: |= 4 when a staged ROI copy did not arrive in time (QI kernel)
+    unsigned *err_flag;   // mapped host word: |= 4 when a staged ROI copy did not arrive in time
+    unsigned copy_polls;  // mbarrier polls before a tile's staged copy counts as late
 };
 
 }  // namespace qtrk

@@ -365,6 +365,7 @@ TrackParams Tracker::Params(int pdt) const
     P.offset_factor = offset_factor_;
     P.gain_factor = gain_factor_;
     P.err_flag = d_err_;
+    P.copy_polls = copy_polls_;
     plan_smem(P);
     return P;
 }
@@ -700,19 +701,24 @@ bool Tracker::IsPinned(const void *p)
     return a.type == cudaMemoryTypeHost;
 }
 
+// What the kernels have flagged since the last call, as warnings.
+void Tracker::ReportErrorsLocked()
+{
+    if (!h_err_ || !*h_err_) return;
+    const unsigned e = *h_err_;
+    *h_err_ = 0;
+    if (e & 3u) Warn("tensor-core Z match: an MMA completion wait timed out; z of the affected ROIs is NaN");
+    if (e & 2u)
+        Warn("tensor-core Z match: the timed-out MMAs had not finished when their tensor-memory columns were "
+             "released; results of that launch are void");
+    if (e & 4u)
+        Warn("a staged ROI copy did not arrive within the wait limit; the ROIs of a late copy are not a number "
+             "(LT_OnlyCOM: void)");
+}
+
 void Tracker::CollectLocked()
 {
-    if (h_err_ && *h_err_) {
-        const unsigned e = *h_err_;
-        *h_err_ = 0;
-        if (e & 3u) Warn("tensor-core Z match: an MMA completion wait timed out; z of the affected ROIs is NaN");
-        if (e & 2u)
-            Warn("tensor-core Z match: the timed-out MMAs had not finished when their tensor-memory columns were "
-                 "released; results of that launch are void");
-        if (e & 4u)
-            Warn("localization kernel: a staged ROI copy did not arrive within the wait limit; results of that "
-                 "launch are void");
-    }
+    ReportErrorsLocked();
     while (!inflight_.empty()) {
         const int idx = inflight_.front();
         Slot &s = slots_[idx];
@@ -973,6 +979,12 @@ void Tracker::SetPixelCalibrationFactors(float offsetFactor, float gainFactor)
     std::lock_guard<std::mutex> lk(mu_);
     offset_factor_ = offsetFactor;
     gain_factor_ = gainFactor;
+}
+
+void Tracker::SetCopyWaitLimit(unsigned polls)
+{
+    std::lock_guard<std::mutex> lk(mu_);
+    copy_polls_ = polls;
 }
 
 // QueuedCPUTracker::ScheduleLocalization, QueuedCPUTracker.cpp:435-456: the ROI rows are copied
@@ -1569,6 +1581,10 @@ std::string Tracker::GetProfileReport()
 
 std::string Tracker::GetWarnings()
 {
+    {
+        std::lock_guard<std::mutex> lk(mu_);  // a caller of the device entries alone collects no batches
+        ReportErrorsLocked();
+    }
     std::lock_guard<std::mutex> lk(warn_mu_);
     std::string w;
     w.swap(warnings_);

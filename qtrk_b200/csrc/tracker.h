@@ -50,6 +50,7 @@ class Tracker : public QueuedTracker {
     void SetLocalizationMode(LocMode_t mode);
     void SetPixelCalibrationImages(const float *offset, const float *gain);
     void SetPixelCalibrationFactors(float offsetFactor, float gainFactor);
+    void SetCopyWaitLimit(unsigned polls);
     void ScheduleLocalization(const void *data, int pitch, int pdt, const LocalizationJob *job);
     int ScheduleFrame(const void *img, int pitch, int width, int height, const ROIPosition *pos, int n, int pdt,
                       const LocalizationJob *job);
@@ -118,6 +119,7 @@ class Tracker : public QueuedTracker {
     void AllocateSlots();
     int AcquireSlotLocked(std::unique_lock<std::mutex> &lk);  // a free slot index (may wait)
     void SubmitLocked(int idx);
+    void ReportErrorsLocked();
     void CollectLocked();            // drain completed slots (FIFO)
     void DrainAllLocked(std::unique_lock<std::mutex> &lk);
     void WaitIdleForReconfigure();
@@ -188,6 +190,7 @@ class Tracker : public QueuedTracker {
     float *d_calib_off_ = nullptr, *d_calib_gain_ = nullptr;
     int calib_count_ = 0;
     float offset_factor_ = 1.0f, gain_factor_ = 1.0f;
+    unsigned copy_polls_ = 1u << 22;
 
     std::mutex mu_;      // slots, queues, LUT state
     std::mutex res_mu_;  // results_

@@ -124,6 +124,10 @@ class QTrkInstance:
         """Scale factors of this instance's calibration images (1, 1 by default)."""
         self.lib.QTrkB200SetPixelCalibrationFactors(self.handle, float(offset_factor), float(gain_factor))
 
+    def SetCopyWaitLimit(self, polls: int) -> None:
+        """Polls for a ROI's staged copy before the ROI is given up (its results are then not a number)."""
+        self.lib.QTrkB200SetCopyWaitLimit(self.handle, int(polls))
+
     # -- LUT building (QTrkInstance.cs:51-60, 95-98) --
     def BeginLUT(self, flags: int | bool = abi.BUILDLUT_NORMALIZE) -> None:
         if isinstance(flags, bool):
