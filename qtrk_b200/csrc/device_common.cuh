@@ -920,7 +920,9 @@ __device__ __forceinline__ float erf_as(float x, float e_mx2)
                 a5 = 1.061405429f, p = 0.3275911f;
     const float sign = x < 0 ? -1.0f : 1.0f;
     const float ax = fabsf(x);
-    const float t = rcp(1.0f + p * ax);
+    // the reciprocal refined once: within rounding of the quotient, which the fit's error shows (4 parameters, 12 to 24
+    // px: as with a division; 1.003-1.024 times that with the unrefined reciprocal). Bounded, as inf * 0 is not a number.
+    const float a = 1.0f + p * fminf(ax, 1e30f), r = rcp(a), t = fmaf(fmaf(-a, r, 1.0f), r, r);
     const float y = 1.0f - (((((a5 * t + a4) * t) + a3) * t + a2) * t + a1) * t * e_mx2;
     return sign * y;
 }
