@@ -65,7 +65,7 @@ struct BlockGroup {
 // kLanes (16 or 32) consecutive lanes of a warp.
 template <int kLanes>
 struct LaneGroup {
-    static constexpr int kFold = 8;
+    static constexpr int kFold = 4;  // 12x12 windows: with 8, COM errors 1.10-1.19 times those of 32 lanes a ROI
     __device__ __forceinline__ unsigned mask() const
     {
         return kLanes == 32 ? 0xffffffffu : ((1u << (kLanes & 31)) - 1u) << (threadIdx.x & 31 & ~(kLanes - 1));
@@ -265,11 +265,36 @@ __device__ __forceinline__ float finish_pixel(float v, int i, int mode, float of
     return v;
 }
 
-// Returns this thread's FP32 partial sums of v and v^2 over the pixels it converted (the first pass
+// Sums of v and v^2 over a thread's pixels. A CTA's threads add their few dozen pixels in FP32; the lanes of a group,
+// which have up to twice as many of a small ROI with 16 lanes as with 32, fold theirs into FP64 after every two.
+template <class G>
+struct PixelSums {
+    static constexpr bool kFolds = G::kFold == 4;
+    float s = 0.0f, s2 = 0.0f;
+    double d = 0.0, d2 = 0.0;
+    __device__ __forceinline__ void add(float v)
+    {
+        s += v;
+        s2 = fmaf(v, v, s2);
+    }
+    __device__ __forceinline__ void fold()  // after every two pixels
+    {
+        if (!kFolds) return;
+        d += (double)s;
+        d2 += (double)s2;
+        s = s2 = 0.0f;
+    }
+    __device__ __forceinline__ double2 total() const
+    {
+        return kFolds ? make_double2(d + (double)s, d2 + (double)s2) : make_double2((double)s, (double)s2);
+    }
+};
+
+// Returns this thread's partial sums of v and v^2 over the pixels it converted (the first pass
 // of CPUTracker::ComputeMeanAndCOM, cpu_tracker.cpp:687-693, so that com_from_sums need not read
 // the tile again for them; callers that do not use them pay nothing once the call is inlined).
 template <class G>
-__device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, int pitch, const TrackParams &P, int bead)
+__device__ inline double2 load_roi(const G &g, float *img, const uint8_t *src, int pitch, const TrackParams &P, int bead)
 {
     const int W = P.width, H = P.height, n = W * H;
     const int bpp = P.pdt == 0 ? 1 : (P.pdt == 1 ? 2 : 4);
@@ -280,7 +305,7 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
     }
     const bool contiguous = pitch == W * bpp && ((reinterpret_cast<uintptr_t>(src) & 15) == 0) &&
                             ((n * bpp) & 15) == 0 && ((reinterpret_cast<uintptr_t>(img) & 15) == 0);
-    float s = 0.0f, s2 = 0.0f;
+    PixelSums<G> sums;
     if (contiguous) {
         // Rows are back to back: the ROI is a run of n/4 chunks of four pixels (4, 8 or 16 input
         // bytes), and chunk c becomes the float4 at img + 4c, so a warp's stores fill 512
@@ -297,14 +322,12 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
                 f.z = finish_pixel(f.z, 4 * c + 2, P.mode, P.offset_factor, P.gain_factor, off, gain);
                 f.w = finish_pixel(f.w, 4 * c + 3, P.mode, P.offset_factor, P.gain_factor, off, gain);
             }
-            s += f.x;
-            s2 = fmaf(f.x, f.x, s2);
-            s += f.y;
-            s2 = fmaf(f.y, f.y, s2);
-            s += f.z;
-            s2 = fmaf(f.z, f.z, s2);
-            s += f.w;
-            s2 = fmaf(f.w, f.w, s2);
+            sums.add(f.x);
+            sums.add(f.y);
+            sums.fold();
+            sums.add(f.z);
+            sums.add(f.w);
+            sums.fold();
             dst[c] = f;
         };
         if (P.pdt == 0) {
@@ -406,29 +429,27 @@ __device__ inline float2 load_roi(const G &g, float *img, const uint8_t *src, in
         }
         g.sync();
         if (!chunked) {
+            int k = 0;
             for (int i = g.rank(); i < n; i += g.size()) {
-                const float v = img[i];
-                s += v;
-                s2 = fmaf(v, v, s2);
+                sums.add(img[i]);
+                if (!(++k & 1)) sums.fold();
             }
         }
         if (chunked) {
             const float4 *img4 = reinterpret_cast<const float4 *>(img);
             for (int c = g.rank(); c < (n >> 2); c += g.size()) {
                 const float4 f = img4[c];
-                s += f.x;
-                s2 = fmaf(f.x, f.x, s2);
-                s += f.y;
-                s2 = fmaf(f.y, f.y, s2);
-                s += f.z;
-                s2 = fmaf(f.z, f.z, s2);
-                s += f.w;
-                s2 = fmaf(f.w, f.w, s2);
+                sums.add(f.x);
+                sums.add(f.y);
+                sums.fold();
+                sums.add(f.z);
+                sums.add(f.w);
+                sums.fold();
             }
         }
     }
     g.sync();
-    return make_float2(s, s2);
+    return sums.total();
 }
 
 // -------------------------------------------------------------------------------------
@@ -447,7 +468,7 @@ struct ComResult {
 // to ~1e-7 relative, far inside the 1e-4 px COM tolerance; for integer pixels the first pass's
 // partial sums, and so the mean, are exact).
 template <class G>
-__device__ ComResult com_from_sums(const G &g, const float *img, int W, int H, float2 part, float bgcorr)
+__device__ ComResult com_from_sums(const G &g, const float *img, int W, int H, double2 part, float bgcorr)
 {
     const int n = W * H, stride = g.size();
     const int dx = stride % W, dy = stride / W;

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(32 * kGaussWarps, kParams == 4 ? 4 : 3)
     const int bead = jobs ? (int)reinterpret_cast<const uint32_t *>(jobs)[(size_t)roi * 6 + 2] : 0;
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
     const LaneGroup<kLanes> lg;
-    const float2 part = load_roi(lg, img, pixels + off, pitch, P, bead);
+    const double2 part = load_roi(lg, img, pixels + off, pitch, P, bead);
     const ComResult com = com_from_sums(lg, img, W, H, part, P.com_bgcorrection);
     float comx = com.x, comy = com.y;
     if (isnan(comx) || isnan(comy)) {  // QueuedCPUTracker.cpp:294-295

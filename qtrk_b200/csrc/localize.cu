@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     BlockGroup g{s.red};
     const int W = P.width, H = P.height;
     float *img = reinterpret_cast<float *>(s.img);
-    const float2 part = load_roi(g, img, pixels + off, pitch, P, bead);
+    const double2 part = load_roi(g, img, pixels + off, pitch, P, bead);
     const ComResult com = com_from_sums(g, img, W, H, part, P.com_bgcorrection);
     float comx = com.x, comy = com.y;
     if (isnan(comx) || isnan(comy)) {  // QueuedCPUTracker.cpp:294-295
