@@ -1055,10 +1055,10 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
     if (skipped) Warn("ScheduleFrame: skipped " + std::to_string(skipped) + " ROI(s) outside the frame");
     if (idx.empty()) return 0;
 
-    // Group ROIs into row bands of at most 32 MiB (or one slot, if smaller); the bands of a frame listed in
-    // scan order keep the caller's order, and one band does. The bands' copies run one after another (each waits for the previous one),
-    // so every band's kernel overlaps the next band's copy and only the last, small band's kernel
-    // is left after the frame has crossed PCIe.
+    // Group ROIs into row bands of at most 32 MiB (or one slot, if smaller). The bands' copies run one after another
+    // on one stream, so every band's kernel overlaps the next band's copy and only the last, small band's kernel
+    // is left after the frame has crossed PCIe. Bands of a frame listed in scan order keep the caller's order, and so
+    // does a single band.
     const size_t band_cap = std::min(slot_bytes_, (size_t)32 << 20);
     const bool pinned = IsPinned(img);
     int minx = width, maxx = 0;
@@ -1069,37 +1069,21 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
     const size_t dpitch = (((size_t)(maxx - minx) * bpp) + 15) & ~(size_t)15;
     auto span_bytes = [&](int y0, int y1) { return (size_t)(y1 - y0) * dpitch; };
     std::vector<std::vector<int>> bands;
+    int top = height, bottom = 0, cuts = 0;  // cuts: bands that a frame of one slot may be cut into; 0: a larger frame
     {
-        int y0 = height, y1 = 0;
         for (int i : idx) {
-            y0 = std::min(y0, pos[i].y);
-            y1 = std::max(y1, pos[i].y + H);
+            top = std::min(top, pos[i].y);
+            bottom = std::max(bottom, pos[i].y + H);
         }
         auto by_row = [&](int a, int b) { return pos[a].y < pos[b].y; };
-        if (span_bytes(y0, y1) <= band_cap && (int)idx.size() <= batch_) {
-            // A frame of several megabytes crosses PCIe in up to three shrinking bands (3:2:1 of its rows), so that
-            // only the last, smallest band's kernel is left after the copy: 1,000 beads of 100x100 u16 in 20 MB,
-            // 582 us per frame in one band, 515 in three or four (the copy alone: 381). Rows that two bands
-            // share are copied twice: they may add at most a tenth. Only for frames listed in scan order,
-            // whose results then come in the same order.
-            int n = 1;
-            if (pinned && span_bytes(y0, y1) >= ((size_t)4 << 20) && std::is_sorted(idx.begin(), idx.end(), by_row))
-                for (n = std::min(3, (int)slots_.size()); n > 1; n--)
-                    if ((size_t)(n - 1) * H * dpitch * 10 <= span_bytes(y0, y1)) break;
-            std::vector<int> cur;
-            const int parts = n * (n + 1) / 2;
-            int part = n;  // share of the rows up to the current band's end
-            for (int i : idx) {
-                const int64_t end = (int64_t)(y1 - y0) * part / parts;
-                if (!cur.empty() && n > 1 && pos[i].y + H - y0 > end) {
-                    bands.push_back(cur);
-                    cur.clear();
-                    n--;
-                    part += n;
-                }
-                cur.push_back(i);
-            }
-            bands.push_back(cur);
+        if (span_bytes(top, bottom) <= band_cap && (int)idx.size() <= batch_) {
+            // A frame of several megabytes may cross PCIe in up to three shrinking bands (see below). Rows that two
+            // bands share are copied twice: they may add at most a tenth. Only for frames listed in scan order, whose
+            // results then come in the same order.
+            cuts = 1;
+            if (pinned && span_bytes(top, bottom) >= ((size_t)4 << 20) && std::is_sorted(idx.begin(), idx.end(), by_row))
+                for (cuts = std::min(3, (int)slots_.size()); cuts > 1; cuts--)
+                    if ((size_t)(cuts - 1) * H * dpitch * 10 <= span_bytes(top, bottom)) break;
         } else {
             std::vector<int> sorted = idx;
             if (!std::is_sorted(sorted.begin(), sorted.end(), by_row))  // frames are usually listed in scan order
@@ -1148,6 +1132,32 @@ int Tracker::ScheduleFrame(const void *img, int pitch, int width, int height, co
         else
             free_.push_back(filling_);
         filling_ = -1;
+    }
+    if (cuts) {
+        // Cut only when nothing is in flight: the frame waits for nobody, and with 3:2:1 of its rows per band only the
+        // last, smallest band's kernel is left after the copy (1,000 beads of 100x100 u16 in 20 MB, one frame at a
+        // time: 649 us in one band, 536 in three; the copy alone: 381). The bands then take free slots at once,
+        // under this lock: no other thread's batch comes between them and no wait can drop the rest. Behind frames
+        // that are still in flight the copy is hidden anyway, and bands cost 4-7 % of the frame rate (the same
+        // frames back to back 457 and 474 us, 1,000 of 64x64 226 and 241).
+        if (cuts > 1) {
+            CollectLocked();
+            if (!inflight_.empty() || (int)free_.size() < cuts) cuts = 1;
+        }
+        std::vector<int> cur;
+        const int parts = cuts * (cuts + 1) / 2;
+        int part = cuts;  // share of the rows up to the current band's end
+        for (int i : idx) {
+            const int64_t end = (int64_t)(bottom - top) * part / parts;
+            if (!cur.empty() && cuts > 1 && pos[i].y + H - top > end) {
+                bands.push_back(cur);
+                cur.clear();
+                cuts--;
+                part += cuts;
+            }
+            cur.push_back(i);
+        }
+        bands.push_back(cur);
     }
     int count = 0;
     for (const std::vector<int> &band : bands) {
