@@ -31,7 +31,8 @@ struct AdjSmem {
     uint32_t *img;        // the tile (tile.cuh)
     double *p, *dx, *dy;  // [nb] profile and its x/y derivatives (normalised in place)
     double *red;          // 32 doubles of reduction scratch
-    double *misc;         // 16 doubles: broadcast values, the last one the mbarrier of the ROI's copy
+    double *misc;         // 16 doubles: broadcast values, the last two the mbarrier of the ROI's copy and copy_late's word
+    __device__ __forceinline__ uint64_t *mbar() const { return reinterpret_cast<uint64_t *>(misc + 14); }
 };
 
 __host__ __device__ inline int adj_smem_bytes(const TrackParams &P, int ts)
@@ -59,19 +60,18 @@ __device__ __forceinline__ AdjSmem adj_view(uint8_t *smem, const TrackParams &P,
     return s;
 }
 
-// Load the ROI's tile; every thread gets the image mean (FP64 sum; asked only where a bin falls back to it). False
-// (for the whole CTA) when the ROI's copy was late.
+// Load the ROI's tile; every thread gets the image mean (FP64 sum; asked only where a bin falls back to it).
 template <int F, int T>
-__device__ __forceinline__ bool adj_load(const AdjSmem &s, const TrackParams &P, int ts, const uint8_t *src, int pitch,
-                                         int bead, float &mean)
+__device__ __forceinline__ float adj_load(const AdjSmem &s, const TrackParams &P, int ts, const uint8_t *src, int pitch,
+                                          int bead)
 {
     const int W = P.width, n = W * P.height;
     uint32_t isum = 0u;
     if (F == kTileF32 && packed_rows(W, ts)) {
+        if (threadIdx.x == 0) copy_late(s.mbar()) = 0u;
         load_roi(BlockGroup{s.red}, reinterpret_cast<float *>(s.img), src, pitch, P, bead);
     } else {
-        const uint8_t *raw = load_raw<F, T>(s.img, ts, P, src, pitch, reinterpret_cast<uint64_t *>(s.misc + 15), [] {});
-        if (!raw) return false;
+        const uint8_t *raw = load_raw<F, T>(s.img, ts, P, src, pitch, s.mbar(), [] {});
         convert_raw<F, T>(s.img, raw, ts, P, bead, isum);
     }
     __syncthreads();
@@ -84,8 +84,7 @@ __device__ __forceinline__ bool adj_load(const AdjSmem &s, const TrackParams &P,
             for (int j = 0; j < 4 && w.x + j < W; j++) v[0] += (double)__uint_as_float(s.img[w.off + j]);
     }
     BlockGroup{s.red}.sum<1>(v);
-    mean = (float)(v[0] / n);
-    return true;
+    return (float)(v[0] / n);
 }
 
 // Profile (and derivatives) at (cx, cy), ROI in the tile: as radial_profile, eight lanes per bin with the direction
@@ -291,16 +290,11 @@ __global__ void __launch_bounds__(kAdjThreads, 8)
     const AdjSmem s = adj_view(smem, P, ts);
     const int bead = beads ? beads[roi] : 0;
     const bool ok = bead >= 0 && bead < P.lut_count && P.lut_planes >= 2;
-    float mean;
-    if (!adj_load<F, kAdjThreads>(s, P, ts, pixels + (int64_t)roi * roi_stride, pitch, ok ? bead : 0, mean)) {
-        if (threadIdx.x == 0)
-            cost[roi] = grad[3 * roi] = grad[3 * roi + 1] = grad[3 * roi + 2] = nanf("");  // nothing to the LUT's
-        return;
-    }
+    const float mean = adj_load<F, kAdjThreads>(s, P, ts, pixels + (int64_t)roi * roi_stride, pitch, ok ? bead : 0);
     const float x = xyz[3 * roi], y = xyz[3 * roi + 1], z = xyz[3 * roi + 2];
     profile_grad<F, kAdjThreads>(s.img, ts, P, x, y, mean, s.p, s.dx, s.dy);
     if (threadIdx.x >= 32) return;
-    if (!ok) {
+    if (!ok || copy_late(s.mbar())) {  // and nothing to the LUT's gradient
         if (threadIdx.x == 0) {
             cost[roi] = nanf("");
             grad[3 * roi] = grad[3 * roi + 1] = grad[3 * roi + 2] = nanf("");
@@ -371,13 +365,9 @@ __global__ void __launch_bounds__(kRefineThreads)
     const int bead = jobs ? jobs[roi].zlutIndex : 0;
     if (bead < 0 || bead >= P.lut_count || P.lut_planes < 2) return;  // no LUT for this ROI: no Z fit to refine
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
+    adj_load<F, kRefineThreads>(s, P, ts, pixels + off, pitch, bead);
     LocalizationResult *res = results + roi;
-    float mean;
-    if (!adj_load<F, kRefineThreads>(s, P, ts, pixels + off, pitch, bead, mean)) {
-        if (threadIdx.x == 0) res->pos.x = res->pos.y = res->pos.z = nanf("");
-        return;
-    }
-    mean = res->imageMean;
+    const float mean = res->imageMean;
     const float x0 = res->pos.x, y0 = res->pos.y;
     float x = x0, y = y0, z = res->pos.z;
     const int nb = P.z_nbins, planes = P.lut_planes;
@@ -435,6 +425,7 @@ __global__ void __launch_bounds__(kRefineThreads)
         if (!taken) break;
     }
     if (threadIdx.x == 0) {
+        if (copy_late(s.mbar())) x = y = z = nanf("");
         res->pos.x = x;
         res->pos.y = y;
         res->pos.z = z;

@@ -34,6 +34,10 @@ struct SmemView {
     float *qrw;  // QI radial weights (qi_nr floats after the twiddles)
     uint8_t *work;
     double *red;
+    __device__ __forceinline__ uint64_t *mbar() const  // of the ROI's copy; copy_late's word behind it
+    {
+        return reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(misc) + 32);
+    }
 };
 
 __device__ __forceinline__ SmemView smem_view(uint8_t *smem, const TrackParams &P)
@@ -228,12 +232,14 @@ __device__ __forceinline__ float z_localize(const SmemView &s, const TrackParams
     radial_profile<F, T>(s.img, P.width, P.height, ts, x, y, mean, nb, P.z_angsteps, P.z_minr, rstep, s.zdirs, prof,
                          (P.mode & kLT_NormalizeProfile) != 0);
     if (P.zprof_f32) {
-        // [hi | lo] BF16 split of the weighted profile: v = hi + lo + O(2^-16 v)
+        // [hi | lo] BF16 split of the weighted profile: v = hi + lo + O(2^-16 v). Of a ROI whose copy was late, not a
+        // number
+        const bool late = copy_late(s.mbar()) != 0u;
         __nv_bfloat16 *pb = static_cast<__nv_bfloat16 *>(P.zprof_bf16) + (size_t)roi * 2 * P.zprof_nbp;
         for (int r = threadIdx.x; r < P.zprof_nbp; r += blockDim.x) {
             float v = 0.0f;
             if (r < nb) {
-                v = prof[r];
+                v = late ? __int_as_float(0x7fc00000) : prof[r];
                 P.zprof_f32[(size_t)roi * nb + r] = v;
                 if (P.z_weights) v *= P.z_weights[r];
             }
@@ -266,11 +272,10 @@ __device__ __forceinline__ float z_localize(const SmemView &s, const TrackParams
 // and 64 us); larger ROIs, five to an SM by their tiles, lose 1 % by it.
 constexpr int kMinBlocks = 7;
 
-// Bring the ROI at `src` into the tile and measure mean and COM; the tables are fetched under the copy. False (for
-// the whole CTA) when the ROI's copy was late.
+// Bring the ROI at `src` into the tile and measure mean and COM; the tables are fetched under the copy.
 template <int F, int T>
-__device__ __forceinline__ bool load_tile(const SmemView &s, const TrackParams &P, const uint8_t *src, int pitch,
-                                          int bead, float bgcorr, ComResult &com)
+__device__ __forceinline__ ComResult load_tile(const SmemView &s, const TrackParams &P, const uint8_t *src, int pitch,
+                                               int bead, float bgcorr)
 {
     const int W = P.width, H = P.height, ts = P.tile_pitch;
     auto tables = [&] {
@@ -278,36 +283,16 @@ __device__ __forceinline__ bool load_tile(const SmemView &s, const TrackParams &
         if (P.sm_zdirs != P.sm_tables) load_z_tables(s, P);
     };
     if (F == kTileF32 && packed_rows(W, ts)) {  // the largest odd ROIs: a tile without room for padded rows
+        if (threadIdx.x == 0) copy_late(s.mbar()) = 0u;
         tables();
         const BlockGroup g{s.red};
         float *img = reinterpret_cast<float *>(s.img);
-        com = com_from_sums(g, img, W, H, load_roi(g, img, src, pitch, P, bead), bgcorr);
-        return true;
+        return com_from_sums(g, img, W, H, load_roi(g, img, src, pitch, P, bead), bgcorr);
     }
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(s.misc) + 32);
-    const uint8_t *raw = load_raw<F, T>(s.img, ts, P, src, pitch, mbar, tables);
-    if (!raw) return false;
+    const uint8_t *raw = load_raw<F, T>(s.img, ts, P, src, pitch, s.mbar(), tables);
     uint32_t isum;
     const double sum = convert_raw<F, T>(s.img, raw, ts, P, bead, isum);
-    com = tile_com<F, T>(s.img, W, H, ts, sum, isum, bgcorr, s.red);
-    return true;
-}
-
-// The result of a ROI whose copy was late: not a number, also in the profile that the tensor-core match would read.
-static __device__ __noinline__ void write_void_result(const TrackParams &P, const LocalizationJob *jobs, int roi,
-                                                      LocalizationResult *results)
-{
-    const float nan = __int_as_float(0x7fc00000);
-    if (P.zprof_f32) {
-        __nv_bfloat16 *pb = static_cast<__nv_bfloat16 *>(P.zprof_bf16) + (size_t)roi * 2 * P.zprof_nbp;
-        for (int r = threadIdx.x; r < 2 * P.zprof_nbp; r += blockDim.x) pb[r] = __float2bfloat16_rn(nan);
-        for (int r = threadIdx.x; r < P.z_nbins; r += blockDim.x) P.zprof_f32[(size_t)roi * P.z_nbins + r] = nan;
-    }
-    if (threadIdx.x == 0) {
-        uint32_t job[6];
-        read_job(jobs, roi, job);
-        write_result(results, roi, job, nan, nan, nan, nan, nan, 1u, nan);
-    }
+    return tile_com<F, T>(s.img, W, H, ts, sum, isum, bgcorr, s.red);
 }
 
 // COM / QI (+ Z): QueuedCPUTracker::ProcessJob (QueuedCPUTracker.cpp:273-361), one CTA of T threads per
@@ -326,11 +311,7 @@ __global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
     // the job's words are read again for the result (no registers held through QI and Z)
     const int bead = jobs ? (int)reinterpret_cast<const uint32_t *>(jobs)[(size_t)roi * 6 + 2] : 0;
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
-    ComResult com;
-    if (!load_tile<F, T>(s, P, pixels + off, pitch, bead, P.com_bgcorrection, com)) {
-        write_void_result(P, jobs, roi, results);
-        return;
-    }
+    const ComResult com = load_tile<F, T>(s, P, pixels + off, pitch, bead, P.com_bgcorrection);
     float comx = com.x, comy = com.y;
     if (isnan(comx) || isnan(comy)) {  // QueuedCPUTracker.cpp:294-295
         comx = (float)(W / 2);
@@ -346,7 +327,12 @@ __global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
     if (threadIdx.x == 0) {
         uint32_t job[6];
         read_job(jobs, roi, job);
-        write_result(results, roi, job, x, y, z, comx, comy, bhit ? 1u : 0u, com.mean);
+        float mean = com.mean;
+        if (copy_late(s.mbar())) {
+            x = y = z = comx = comy = mean = __int_as_float(0x7fc00000);
+            bhit = true;
+        }
+        write_result(results, roi, job, x, y, z, comx, comy, bhit ? 1u : 0u, mean);
     }
 }
 
@@ -365,6 +351,7 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
     read_job(jobs, roi, job);
     const int bead = (int)job[2];
     const int64_t off = roi_offsets ? roi_offsets[roi] : (int64_t)roi * roi_stride;
+    if (threadIdx.x == 0) copy_late(s.mbar()) = 0u;
     BlockGroup g{s.red};
     const int W = P.width, H = P.height;
     float *img = reinterpret_cast<float *>(s.img);
@@ -412,13 +399,7 @@ __global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
     const int bead = blockIdx.x;
     if (bead >= nbeads) return;
     const SmemView s = smem_view(smem, P);
-    const int nb = P.z_nbins;
-    float *dst = lut + ((size_t)bead * P.lut_planes + plane) * nb;
-    ComResult com;
-    if (!load_tile<F, T>(s, P, pixels + (size_t)pitch * P.height * bead, pitch, bead, 0.0f, com)) {
-        for (int r = threadIdx.x; r < nb; r += T) dst[r] = __int_as_float(0x7fc00000);  // a row that no match takes
-        return;
-    }
+    const ComResult com = load_tile<F, T>(s, P, pixels + (size_t)pitch * P.height * bead, pitch, bead, 0.0f);
     float x, y, mean = 0.0f;
     if (known_pos) {
         x = known_pos[bead].x;
@@ -430,6 +411,7 @@ __global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
         bool bhit;
         qi_localize<F, T>(s, P, mean, x, y, bhit, nullptr);
     }
+    const int nb = P.z_nbins;
     float *prof = reinterpret_cast<float *>(s.work);
     const float rstep = (P.z_maxr - P.z_minr) / (float)nb;
     __syncthreads();
@@ -439,7 +421,9 @@ __global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
     }
     radial_profile<F, T>(s.img, P.width, P.height, P.tile_pitch, x, y, mean, nb, P.z_angsteps, P.z_minr, rstep, s.zdirs,
                          prof, normalize != 0);
-    for (int r = threadIdx.x; r < nb; r += T) dst[r] += prof[r];
+    float *dst = lut + ((size_t)bead * P.lut_planes + plane) * nb;
+    const bool late = copy_late(s.mbar()) != 0u;  // not a number: a row that no match takes
+    for (int r = threadIdx.x; r < nb; r += T) dst[r] = late ? __int_as_float(0x7fc00000) : dst[r] + prof[r];
 }
 
 // QueuedCPUTracker::FinalizeLUT (QueuedCPUTracker.cpp:648-659): NormalizeRadialProfile
