@@ -336,9 +336,11 @@ __global__ void __launch_bounds__(T, T == 128 ? kMinBlocks : (T == 256 ? 2 : 1))
     }
 }
 
-// 2D Gaussian MLE (+ Z) for ROIs above 32x32 or with QI/Z bits: one CTA per ROI on a plain tile.
-// Kept apart from the QI kernel so that its register budget is free of the MLE's FP64 solve.
-__global__ void __launch_bounds__(kBlockThreads, kMinBlocks)
+// 2D Gaussian MLE (+ Z) for ROIs above 32x32 or with the Z bit: one CTA per ROI on a plain tile.
+// Kept apart from the QI kernel, whose registers are not the MLE's. kBlocks: CTAs per SM it is compiled for, see
+// gauss_cta_kernel.
+template <int kBlocks>
+__global__ void __launch_bounds__(kBlockThreads, kBlocks)
     localize_gauss_kernel(TrackParams P, const uint8_t *__restrict__ pixels, int pitch, int64_t roi_stride,
                           const int64_t *__restrict__ roi_offsets, const LocalizationJob *__restrict__ jobs, int count,
                           LocalizationResult *__restrict__ results)
@@ -532,6 +534,17 @@ static int wide_cta(const TrackParams &P, int count)
     return 0;
 }
 
+// The Gaussian kernel by the CTAs per SM that it is compiled for: seven (72 registers, some spills), except for the 20
+// FP32 sums of the 5-parameter form where an SM's shared memory holds no more than five CTAs anyway (96 registers). f32,
+// compiled for seven and five: 4 parameters, 4,000 x 40x40 408 and 466 us, 2,000 x 64x64 426 and 472, 100x100 970 and
+// 964; 5 parameters, 40x40 426 and 459, 2,000 x 88x88 (six fit) 544 and 551, 92x92 (five fit) 569 and 554, 100x100 721
+// and 704, 150x150 1839 and 1768.
+static QiKernel gauss_cta_kernel(const TrackParams &P)
+{
+    const bool five = (P.mode & kLT_Gaussian5P) && (228 * 1024) / (P.smem_bytes + 1024) <= 5;
+    return five ? localize_gauss_kernel<5> : localize_gauss_kernel<7>;
+}
+
 static bool g_attrs_set[64];
 
 cudaError_t prepare_kernels(int device)
@@ -548,8 +561,10 @@ cudaError_t prepare_kernels(int device)
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)))
                 return e;
         }
-    if ((e = cudaFuncSetAttribute(localize_gauss_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)))
-        return e;
+    for (QiKernel k : {localize_gauss_kernel<5>, localize_gauss_kernel<7>})
+        if ((e = cudaFuncSetAttribute(reinterpret_cast<const void *>(k), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kMaxSmem)))
+            return e;
     if ((e = cudaFuncSetAttribute(profile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem))) return e;
     if ((e = prepare_gauss_kernels())) return e;
     g_attrs_set[device] = true;
@@ -566,8 +581,8 @@ cudaError_t launch_localize(const TrackParams &P, const uint8_t *pixels, int pit
     if (use_gauss_warp(P))
         return launch_gauss_warp(P, pixels, pitch, roi_stride, roi_offsets, jobs, count, results, stream);
     if ((P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI)) {
-        localize_gauss_kernel<<<count, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, roi_stride,
-                                                                              roi_offsets, jobs, count, results);
+        gauss_cta_kernel(P)<<<count, kBlockThreads, P.smem_bytes, stream>>>(P, pixels, pitch, roi_stride, roi_offsets,
+                                                                           jobs, count, results);
     } else {
         const int wide = wide_cta(P, count);
         kQiKernels[tile_format(P, P.tile_pitch)][wide]<<<count, kBlockThreads << wide, P.smem_bytes, stream>>>(
@@ -658,7 +673,7 @@ void localize_node(const TrackParams &P, int count, cudaKernelNodeParams &kp)
     } else {
         const bool gauss = (P.mode & kLT_Gaussian2D) && !(P.mode & kLT_QI);
         const int wide = gauss ? 0 : wide_cta(P, count);
-        kp.func = gauss ? reinterpret_cast<void *>(localize_gauss_kernel)
+        kp.func = gauss ? reinterpret_cast<void *>(gauss_cta_kernel(P))
                         : reinterpret_cast<void *>(kQiKernels[tile_format(P, P.tile_pitch)][wide]);
         kp.gridDim = dim3(count);
         kp.blockDim = dim3(kBlockThreads << wide);
