@@ -607,7 +607,7 @@ __device__ inline void warp_fft(float2 *buf, int L, int log2L, const float2 *tw,
 // FFT(reverse(p))* = e^{-2 pi i k/L} FFT(p) for real p, the product the reference forms
 // from two forward FFTs equals e^{-2 pi i k/L} P[k]^2, so one forward and one inverse
 // FFT per iteration give both axes. Result: ac[n] = (out_x[n], out_y[n]). A holds the packed
-// profile in bit-reversed order on entry (as qi_profiles_sym writes it). Warp 0 only.
+// profile in bit-reversed order on entry (as qi_profiles writes it). Warp 0 only.
 __device__ inline void qi_autoconv_fft_filled(int nr, float2 *A, float2 *ac, const float2 *tw)
 {
     const int lane = threadIdx.x & 31;

@@ -15,7 +15,7 @@
 // is left per iteration: the sums across lanes, the divisions and the 5x5 solve.
 //
 // What bounds it: instruction issue (75 % used at 24-32 warps per SM). Measured on 100,000 16x16 f32
-// ROIs, 8 iterations: 4 parameters 1.520 -> 0.403 ms, 5 parameters (20,000 15x15 u16) 0.434 -> 0.137 ms
+// ROIs, 8 iterations: 4 parameters 1.520 -> 0.404 ms, 5 parameters (20,000 15x15 u16) 0.434 -> 0.136 ms
 // against one warp per ROI with every pixel forming all its products in FP32 and adding eight (or twenty)
 // sums; one warp per ROI with the column factors taken out reached 0.613 and 0.232 ms.
 #include <cstdint>
@@ -438,8 +438,8 @@ __global__ void __launch_bounds__(32 * kGaussWarps, 4)
 using GaussKernel = void (*)(TrackParams, const uint8_t *, int, int64_t, const int64_t *, const LocalizationJob *, int,
                              LocalizationResult *);
 
-// Two ROIs per warp as long as a row fits half a warp (16x16: 0.456 ms with 16 lanes per ROI, 0.613 ms with
-// 32); wider rows would need two passes over the columns per step.
+// Two ROIs per warp as long as a row fits half a warp (16x16, 4 parameters: 0.404 ms with 16 lanes per ROI;
+// 0.456 with 16 and 0.613 with 32 before the reciprocals became one instruction); wider rows would need two passes over the columns per step.
 int gauss_lanes_per_roi(const TrackParams &P) { return P.width <= 16 ? 16 : 32; }
 
 GaussKernel gauss_kernel_for(const TrackParams &P)

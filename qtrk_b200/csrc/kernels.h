@@ -12,8 +12,8 @@ namespace qtrk {
 void plan_smem(TrackParams &P);
 // Raise the dynamic shared-memory limit of the kernels once per device.
 cudaError_t prepare_kernels(int device);
-// The Gaussian-only mode on ROIs of at most 32x32 pixels (gauss.cu, one warp per ROI): whether it
-// serves P, its launch, and its graph node (function, grid, block, shared memory).
+// The Gaussian-only mode on ROIs of at most 32x32 pixels (gauss.cu, half a warp per ROI of up to 16
+// columns, else one warp): whether it serves P, its launch, and its graph node (function, grid, block, shared memory).
 bool use_gauss_warp(const TrackParams &P);
 cudaError_t prepare_gauss_kernels();
 void gauss_warp_node(const TrackParams &P, int count, cudaKernelNodeParams &kp);

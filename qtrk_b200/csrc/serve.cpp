@@ -389,7 +389,9 @@ void Server::LaunchBatch(Lane &lane, Tracker *t, const std::vector<Request *> &b
         lane.a_count = m[b + 1] - m[b];
         lane.a_res = lane.d_res + m[b];
         cudaKernelNodeParams kp;
-        localize_node(P, lane.a_count, kp);  // same function and shared memory as the graph's node
+        // the whole node is replaced at every replay: function and block size follow the band's count and the
+        // calibration images, which the graph's key does not hold
+        localize_node(P, lane.a_count, kp);
         kp.kernelParams = lane.args;          // the argument values are copied here
         ck(cudaGraphExecKernelNodeSetParams(g.exec, g.kernel[b], &kp), "cudaGraphExecKernelNodeSetParams");
     }

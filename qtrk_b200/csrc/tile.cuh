@@ -16,7 +16,10 @@
 //
 // Results also do not depend on T (the launcher picks T by the number of ROIs): whatever is summed in FP32 is
 // cut into pieces that are the same for every T (the eight direction subsets of a circle, the 512 pixel
-// chains of the COM), and the pieces meet in the same order or in FP64.
+// chains of the COM), and the pieces meet in the same order or in FP64. FP64 sums across threads (the COM's moments, a
+// float ROI's mean) are formed in an order that follows T. They are exact, and so the same, as long as no pixel is
+// negative: a moment's terms are then multiples of 2^-25 of the mean, and their sum stays below 2^53 of that unit.
+// With negative pixels they agree to FP64 rounding (1e-16), far below the FP32 result's.
 #pragma once
 #include "bulk_copy.cuh"
 #include "device_common.cuh"
@@ -771,7 +774,7 @@ __device__ __forceinline__ void qi_profiles(const uint32_t *img, int W, int H, i
             sm[2] = s02[0].y;
             sm[3] = s31[0].x;
         } else {
-            // bilinear()'s rule per coordinate: a sample is inside when -1 < x < W-1 and
+            // the rule of Interpolate (utils.h:40-58) per coordinate: a sample is inside when -1 < x < W-1 and
             // -1 < y < H-1, and its cell starts at the truncation of max(x, 0)
             const float xhi = (float)(W - 1), yhi = (float)(H - 1);
             float s2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
