@@ -438,8 +438,9 @@ __global__ void __launch_bounds__(32 * kGaussWarps, 4)
 using GaussKernel = void (*)(TrackParams, const uint8_t *, int, int64_t, const int64_t *, const LocalizationJob *, int,
                              LocalizationResult *);
 
-// Two ROIs per warp as long as a row fits half a warp (16x16, 4 parameters: 0.404 ms with 16 lanes per ROI;
-// 0.456 with 16 and 0.613 with 32 before the reciprocals became one instruction); wider rows would need two passes over the columns per step.
+// Two ROIs per warp as long as a row fits half a warp (16x16, 4 parameters: 0.404 ms with 16 lanes per ROI; 0.456 with
+// 16 and 0.613 with 32 before the reciprocals became one instruction); wider rows would need two passes over the
+// columns per step.
 int gauss_lanes_per_roi(const TrackParams &P) { return P.width <= 16 ? 16 : 32; }
 
 GaussKernel gauss_kernel_for(const TrackParams &P)

@@ -16,10 +16,10 @@
 //
 // Results also do not depend on T (the launcher picks T by the number of ROIs): whatever is summed in FP32 is
 // cut into pieces that are the same for every T (the eight direction subsets of a circle, the 512 pixel
-// chains of the COM), and the pieces meet in the same order or in FP64. FP64 sums across threads (the COM's moments, a
-// float ROI's mean) are formed in an order that follows T. They are exact, and so the same, as long as no pixel is
-// negative: a moment's terms are then multiples of 2^-25 of the mean, and their sum stays below 2^53 of that unit.
-// With negative pixels they agree to FP64 rounding (1e-16), far below the FP32 result's.
+// chains of the COM), and the pieces meet in the same order or in FP64. FP64 sums across threads are formed in an order
+// that follows T. Those of the COM's moments are exact, and so the same, as long as no pixel is negative: their
+// terms are then multiples of 2^-25 of the mean, and a sum stays below 2^53 of that unit. Moments with negative
+// pixels, and a float ROI's mean, agree to FP64 rounding (1e-16), far below that of the FP32 result.
 #pragma once
 #include "bulk_copy.cuh"
 #include "device_common.cuh"
