@@ -599,7 +599,8 @@ __global__ void __launch_bounds__(1024, 1) com_warp_kernel(TrackParams P, const 
 // exactly for the mean.
 // What bounds it: instruction issue. Per 8 pixels pass 2 takes about 40 instructions (load, unpacking, |v - mean|,
 // sums) where the walk over 16-byte chunks took 53: 10,000 x 100x100 u16 55.8 -> 46.9 us (65 % of the measured copy
-// rate, 54 % before), 8,000 x 100x100 f32 72.4 -> 52.8 us (92 %).
+// rate, 54 % before), 8,000 x 100x100 f32 72.4 -> 52.8 us (92 %), in steady repetition; the first pass over a new stack
+// takes as long as the walk's.
 template <int PDT>
 __global__ void __launch_bounds__(640, 2) com_column_kernel(TrackParams P, const uint8_t *__restrict__ pixels,
                                                              int64_t roi_stride, const LocalizationJob *__restrict__ jobs,
